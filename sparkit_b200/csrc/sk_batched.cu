@@ -39,11 +39,27 @@ struct sk_batch_s {
   void* ws = nullptr;
   size_t ws_bytes = 0;
   int* counter = nullptr;
+  // Sliced copy of the systems that the cluster kernel solves: system s has
+  // slices cl_slice0[s] .. of 32 rows each, slice t padded to its longest row
+  // and stored slot by slot (entry k of lane l at cl_off[t] + 32 k + l) with
+  // 16-bit columns inside the system; cl_len holds each row's length.
+  int* cl_slice0 = nullptr;
+  int* cl_off = nullptr;
+  unsigned char* cl_len = nullptr;
+  unsigned short* cl_col = nullptr;
+  float* cl_val = nullptr;
+  int* cl_order = nullptr;  // per class: its systems, longest first, then the systems left to batched_cg_kernel
+  std::vector<int> cl_first;            // first entry of each class in cl_order, and the end
+  std::vector<std::vector<int>> cl_at;  // per class: its systems' positions in `order`, ascending
+  int cl_ctas[8] = {};  // per class: CTAs in flight
+  cudaStream_t fork[8] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[8] = {};
   // cached graph of the last solve
   cudaGraphExec_t graph = nullptr;
   const void* graph_key[4] = {nullptr, nullptr, nullptr, nullptr};
   int graph_variant = -1;
   int graph_ctas = 0;
+  sk::i64 graph_launches = 0;
   sk_batch_config graph_cfg{};
 };
 
@@ -296,6 +312,331 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batched_cg_kernel(BatchView bv,
   }
 }
 
+// ------------------------------------------------------------------
+// One system per thread-block cluster
+//
+// batched_cg_kernel keeps one system on one CTA and its vectors in global
+// memory: 1024 systems of 1k to 64k rows have 300 of them in flight, whose
+// matrices and vectors exceed the L2 many times over, so every iteration
+// reads them from HBM again.  Here a cluster of C CTAs owns a system for its
+// whole solve: each CTA keeps its rows' five FP32 vectors in shared memory
+// (20 bytes a row), gathers p from there (from the neighbour CTA's shared
+// memory for a column outside its rows) and streams only the matrix, 6 bytes
+// an entry, which stays in L2 because few systems are in flight.  A dot
+// product is one exchange of partial sums through shared memory and one
+// cluster barrier; nothing waits in a loop.
+//
+// Row sums have the bits of batched_cg_kernel<1, NT> (FP32, storage order);
+// the dot products' partial sums meet in another order.
+//
+// 1024 systems of 1k to 64k rows (2-D and 3-D grids, sizes log-uniform): 105 ms with one CTA per system, 18.1 ms so.  Systems of more than
+// 65,536 rows (16-bit columns) or rows of more than 64 entries stay with
+// batched_cg_kernel, as do two or more lanes per row.
+// ------------------------------------------------------------------
+struct ClusterView {
+  const int* sys_off;
+  const int* order;  // this launch's systems
+  int count;
+  const int* slice0;
+  const int* off;
+  const unsigned char* len;
+  const unsigned short* col;
+  const float* val;
+  int cap;  // rows a CTA's shared memory holds
+};
+
+constexpr int kClE = 8;        // entries of a row loaded together
+constexpr int kClMaxLen = 64;  // longest row of the sliced copy
+constexpr i64 kClMaxRows = 65536;
+
+__device__ __forceinline__ unsigned cl_smem(const void* p) { return static_cast<unsigned>(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ unsigned cl_map(unsigned addr, unsigned rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float cl_ldf(unsigned addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ void cl_std(unsigned addr, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(addr), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cl_sti(unsigned addr, int v) {
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+template <int C>
+__device__ __forceinline__ void cl_barrier() {
+  if constexpr (C == 1) {
+    __syncthreads();
+  } else {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+  }
+}
+
+struct ClRed {
+  double part[2][32][2];  // a CTA's warp sums
+  double slot[2][8][2];   // the cluster's CTA sums
+};
+
+// The cluster-wide sums of v, the same bits in every thread: warp trees, a
+// tree over the CTA's warps, then the CTAs in rank order.  Successive calls
+// alternate the two sets, so one barrier a call is enough.
+template <int C, int NT, int NR>
+__device__ __forceinline__ void cl_sum(double (&v)[NR], ClRed& m, int& set, unsigned rank) {
+  constexpr int W = NT / 32;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  warp_reduce<NR>(v);
+  if (lane == 0)
+#pragma unroll
+    for (int j = 0; j < NR; ++j) m.part[set][warp][j] = v[j];
+  __syncthreads();
+  if (C == 1 || warp == 0) {
+#pragma unroll
+    for (int j = 0; j < NR; ++j) v[j] = lane < W ? m.part[set][lane][j] : 0.0;
+    warp_reduce<NR>(v);
+  }
+  if constexpr (C > 1) {
+    if (warp == 0 && lane < C) {
+      const unsigned to = cl_map(cl_smem(&m.slot[set][rank][0]), lane);
+#pragma unroll
+      for (int j = 0; j < NR; ++j) cl_std(to + 8 * j, v[j]);
+    }
+    cl_barrier<C>();
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
+      double t = 0.0;
+#pragma unroll
+      for (int c = 0; c < C; ++c) t += m.slot[set][c][j];
+      v[j] = t;
+    }
+  }
+  set ^= 1;
+}
+
+template <int C, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB) batched_cluster_kernel(ClusterView cv, BatchArgs ar, int* counter) {
+  extern __shared__ __align__(16) float cl_vec[];
+  __shared__ ClRed red;
+  __shared__ int s_q[2];
+  float* p = cl_vec;
+  float* r = p + cv.cap;
+  float* dinv = r + cv.cap;
+  float* d = dinv + cv.cap;  // d and q together hold the FP64 residual between two inner solves
+  float* q = d + cv.cap;
+  double* r64 = reinterpret_cast<double*>(d);
+  int* s_off = reinterpret_cast<int*>(q + cv.cap);  // where each slice and how long each row is
+  unsigned char* s_len = reinterpret_cast<unsigned char*>(s_off + cv.cap / 32);
+  const int tid = threadIdx.x, lane = tid & 31;
+  unsigned rank = 0;
+  if constexpr (C > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const unsigned p_addr = cl_smem(p);
+  int set = 0;
+  for (int turn = 0;; turn ^= 1) {
+    if (rank == 0 && tid == 0) {
+      const int t = atomicAdd(counter, 1);
+      if constexpr (C == 1) {
+        s_q[turn] = t;
+      } else {
+        for (int c = 0; c < C; ++c) cl_sti(cl_map(cl_smem(&s_q[turn]), c), t);
+      }
+    }
+    cl_barrier<C>();
+    const int qi = s_q[turn];
+    if (qi >= cv.count) break;
+    const int sys = cv.order[qi];
+    const int r0 = cv.sys_off[sys];
+    const int n = cv.sys_off[sys + 1] - r0;
+    // this CTA's rows of the system: [my0, my0 + cnt), whole slices
+    const unsigned per = max(32, (((n + C - 1) / C) + 31) & ~31);
+    const unsigned my0 = rank * per;
+    const int cnt = max(0, min(static_cast<int>(per), n - static_cast<int>(my0)));
+    const unsigned magic = 0xffffffffu / per + 1;  // j / per = umulhi(j, magic) for j < 65536
+    const int slice0 = cv.slice0[sys] + static_cast<int>(my0 >> 5);
+    const double* b = ar.b + r0 + my0;
+    double* x = ar.x + r0;
+    auto row = [&](int i, int& len, int& at) {
+      len = s_len[i];
+      at = s_off[i >> 5] + lane;
+    };
+    for (int i = tid; i < cnt; i += NT) s_len[i] = __ldg(cv.len + (static_cast<i64>(slice0) << 5) + i);
+    for (int i = tid; i < (cnt + 31) >> 5; i += NT) s_off[i] = __ldg(cv.off + slice0 + i);
+    __syncthreads();
+    // Jacobi: inverse diagonal in FP32; ||b|| in FP64
+    double nb[1] = {0.0};
+    for (int i = tid; i < cnt; i += NT) {
+      int len, at;
+      row(i, len, at);
+      float dg = 0.0f;
+      for (int k = 0; k < len; ++k)
+        if (__ldg(cv.col + at + 32 * k) == my0 + i) dg = __ldg(cv.val + at + 32 * k);
+      dinv[i] = dg != 0.0f ? static_cast<float>(1.0 / static_cast<double>(dg)) : 0.0f;
+      nb[0] += b[i] * b[i];
+    }
+    cl_sum<C, NT, 1>(nb, red, set, rank);
+    const double bnorm = sqrt(nb[0]);
+    int inner_total = 0, outer = 0, conv = 0;
+    double rel = 0.0;
+    if (bnorm == 0.0) {
+      for (int i = tid; i < cnt; i += NT) x[my0 + i] = 0.0;
+      conv = 1;
+    } else {
+      for (;; ++outer) {
+        // r64 = b - A x in FP64 (FP32 values promoted exactly)
+        double rr[1] = {0.0};
+        for (int i = tid; i < cnt; i += NT) {
+          int len, at;
+          row(i, len, at);
+          double ax = 0.0;
+          for (int k = 0; k < len; ++k)
+            ax += static_cast<double>(__ldg(cv.val + at + 32 * k)) * __ldcg(x + __ldg(cv.col + at + 32 * k));
+          const double ri = b[i] - ax;
+          r64[i] = ri;
+          rr[0] += ri * ri;
+        }
+        cl_sum<C, NT, 1>(rr, red, set, rank);
+        const double rn = sqrt(rr[0]);
+        rel = rn / bnorm;
+        if (rel < ar.tol) {
+          conv = 1;
+          break;
+        }
+        if (outer >= ar.max_outer) break;
+        double itol = ar.inner_tol;
+        const double needed = ar.tol / rel;
+        if (ar.adaptive && 0.5 * needed < itol) itol = fmax(0.5 * needed, 1e-7);
+        // inner FP32 Jacobi-CG on A d = r / ||r||, d0 = 0
+        const double inv = 1.0 / rn;
+        double t2[2] = {0.0, 0.0};
+        for (int i = tid; i < cnt; i += NT) {
+          const float ri = static_cast<float>(r64[i] * inv);
+          const float zi = __fmul_rn(dinv[i], ri);
+          r[i] = ri;
+          p[i] = zi;
+          t2[0] += static_cast<double>(__fmul_rn(ri, ri));
+          t2[1] += static_cast<double>(__fmul_rn(ri, zi));
+        }
+        cl_sum<C, NT, 2>(t2, red, set, rank);  // every r64 read before d is written, p complete
+        for (int i = tid; i < cnt; i += NT) d[i] = 0.0f;
+        const float r0n = sqrtf(static_cast<float>(t2[0]));
+        float rz = static_cast<float>(t2[1]);
+        for (int it = 0; it < ar.max_inner; ++it) {
+          // q = A p, <p, q>
+          double pq[1] = {0.0};
+          for (int i = tid; i < cnt; i += NT) {
+            int len, at;
+            row(i, len, at);
+            float sum = 0.0f;
+            for (int k0 = 0; k0 < len; k0 += kClE) {
+              unsigned c[kClE];
+              float w[kClE], xv[kClE];
+              bool mine = true;
+#pragma unroll
+              for (int j = 0; j < kClE; ++j) {
+                const bool in = k0 + j < len;
+                c[j] = in ? __ldg(cv.col + at + 32 * (k0 + j)) : my0;
+                w[j] = in ? __ldg(cv.val + at + 32 * (k0 + j)) : 0.0f;
+              }
+              if constexpr (C > 1) {
+#pragma unroll
+                for (int j = 0; j < kClE; ++j) mine = mine && c[j] - my0 < per;
+              }
+              if (C == 1 || mine) {
+#pragma unroll
+                for (int j = 0; j < kClE; ++j) xv[j] = p[c[j] - my0];
+              } else {
+#pragma unroll
+                for (int j = 0; j < kClE; ++j) {
+                  const unsigned own = __umulhi(c[j], magic);
+                  xv[j] = cl_ldf(cl_map(p_addr + 4 * (c[j] - own * per), own));
+                }
+              }
+#pragma unroll
+              for (int j = 0; j < kClE; ++j)
+                if (k0 + j < len) sum = __fadd_rn(sum, __fmul_rn(w[j], xv[j]));
+            }
+            q[i] = sum;
+            pq[0] += static_cast<double>(__fmul_rn(p[i], sum));
+          }
+          cl_sum<C, NT, 1>(pq, red, set, rank);
+          const float alpha = rz / static_cast<float>(pq[0]);
+          double s2[2] = {0.0, 0.0};
+#pragma unroll 4
+          for (int i = tid; i < cnt; i += NT) {
+            d[i] = __fadd_rn(__fmul_rn(alpha, p[i]), d[i]);
+            const float ri = __fsub_rn(r[i], __fmul_rn(alpha, q[i]));
+            r[i] = ri;
+            s2[0] += static_cast<double>(__fmul_rn(ri, ri));
+            s2[1] += static_cast<double>(__fmul_rn(ri, __fmul_rn(dinv[i], ri)));
+          }
+          cl_sum<C, NT, 2>(s2, red, set, rank);
+          ++inner_total;
+          if (sqrtf(static_cast<float>(s2[0])) / r0n < static_cast<float>(itol)) break;
+          const float rz_new = static_cast<float>(s2[1]);
+          const float beta = rz_new / rz;
+          rz = rz_new;
+#pragma unroll 4
+          for (int i = tid; i < cnt; i += NT) p[i] = __fadd_rn(__fmul_rn(dinv[i], r[i]), __fmul_rn(beta, p[i]));
+          cl_barrier<C>();  // p complete
+        }
+        for (int i = tid; i < cnt; i += NT) x[my0 + i] += rn * static_cast<double>(d[i]);
+        cl_barrier<C>();  // x complete, d read
+      }
+    }
+    if (rank == 0 && tid == 0) {
+      ar.inner_its[sys] = inner_total;
+      ar.outer_its[sys] = outer;
+      ar.rel_res[sys] = rel;
+      ar.converged[sys] = conv;
+    }
+  }
+}
+
+// The sliced copy: one CTA per system, a warp per slice.
+__global__ void cl_fill_kernel(BatchView bv, const int* __restrict__ slice0, const int* __restrict__ off,
+                               unsigned char* __restrict__ len, unsigned short* __restrict__ col,
+                               float* __restrict__ val) {
+  const int sys = blockIdx.x, lane = threadIdx.x & 31;
+  const int r0 = bv.sys_off[sys], n = bv.sys_off[sys + 1] - r0;
+  const int s0 = slice0[sys], s1 = slice0[sys + 1];
+  for (int s = s0 + (threadIdx.x >> 5); s < s1; s += blockDim.x >> 5) {
+    const int i = 32 * (s - s0) + lane;
+    const int a = i < n ? bv.rp[r0 + i] : 0, l = i < n ? bv.rp[r0 + i + 1] - a : 0;
+    len[(static_cast<i64>(s) << 5) + lane] = static_cast<unsigned char>(l);
+    for (int k = 0; k < l; ++k) {
+      col[off[s] + 32 * k + lane] = static_cast<unsigned short>(bv.col[a + k] - r0);
+      val[off[s] + 32 * k + lane] = bv.val[a + k];
+    }
+  }
+}
+
+using ClusterFn = void (*)(ClusterView, BatchArgs, int*);
+
+// Classes of systems by rows, the smallest cluster whose shared memory holds
+// them: `cap` rows of 21 bytes and a slice's offset per 32 of them a CTA.
+struct ClusterClass {
+  int C, NT, cap;
+  ClusterFn fn;
+  size_t smem() const { return static_cast<size_t>(cap) * 21 + static_cast<size_t>(cap) / 8; }
+};
+const ClusterClass kClasses[] = {
+    {1, 512, 5376, batched_cluster_kernel<1, 512, 2>},
+    {1, 1024, 10848, batched_cluster_kernel<1, 1024, 1>},
+    {2, 1024, 10848, batched_cluster_kernel<2, 1024, 1>},
+    {4, 1024, 10848, batched_cluster_kernel<4, 1024, 1>},
+    {8, 1024, 10848, batched_cluster_kernel<8, 1024, 1>},
+};
+constexpr int kNumClasses = sizeof(kClasses) / sizeof(kClasses[0]);
+
+int class_of(i64 n) {
+  if (n > kClMaxRows) return kNumClasses;
+  for (int c = 0; c < kNumClasses; ++c)
+    if (n <= static_cast<i64>(kClasses[c].C) * kClasses[c].cap) return c;
+  return kNumClasses;
+}
+
 using KernelFn = void (*)(BatchView, BatchArgs);
 
 struct Variant {
@@ -327,7 +668,8 @@ int ctas_for(const sk_batch_s* B, const Variant& v) {
   return per_sm * B->sm_count;
 }
 
-sk_status ensure_batch_ws(sk_batch_s* B, int ctas) {
+sk_status ensure_batch_ws(sk_batch_s* B, const Variant& v, int ctas) {
+  if (v.G == 1 && B->cl_val && B->cl_at.back().empty()) return SK_OK;  // every system runs in shared memory
   const i64 slot32 = 5 * (B->nmax + 64);
   const i64 slot64 = B->nmax + 64;
   const size_t need = static_cast<size_t>(ctas) * (slot32 * 4 + slot64 * 8) + 4096;
@@ -369,6 +711,167 @@ BatchArgs make_args(sk_batch_s* B, int ctas, const double* b, double* x, const s
 
 BatchView view_of(const sk_batch_s* B) {
   return BatchView{B->sys_off, B->order, B->row_ptr, B->col, B->vals, static_cast<int>(B->nsys)};
+}
+
+// CTAs of a class in flight at once, in whole clusters; 0 when the device
+// cannot run it.
+int cluster_ctas(const ClusterClass& k) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  cfg.gridDim = dim3(static_cast<unsigned>(k.C));
+  cfg.blockDim = dim3(static_cast<unsigned>(k.NT));
+  cfg.dynamicSmemBytes = k.smem();
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(k.C);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(k.smem())) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, k.fn, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return clusters * k.C;
+}
+
+// Enqueues the solve of the first `limit` systems of the queue on B->stream:
+// with one lane per row each class of the sliced copy as its own launch, the
+// classes side by side (the widest clusters first, so that the CTAs of the
+// narrow ones fill in behind them), and the systems that no class takes, or
+// all of them with several lanes per row, as one batched_cg_kernel launch.
+sk_status enqueue_batch(sk_batch_s* B, const Variant& v, int ctas, BatchArgs a, int limit) {
+  BatchView bv = view_of(B);
+  cudaStream_t st = B->stream;
+  SK_CUDA(cudaMemsetAsync(B->counter, 0, 64, st));
+  if (v.G != 1 || !B->cl_val) {
+    a.limit = limit;
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    v.fn<<<std::min(ctas, limit), v.NT, 0, st>>>(bv, a);
+    return SK_OK;
+  }
+  auto taken = [&](int k) {  // systems of class k among the first `limit`
+    const auto& at = B->cl_at[static_cast<size_t>(k)];
+    return static_cast<int>(std::lower_bound(at.begin(), at.end(), limit) - at.begin());
+  };
+  SK_CUDA(cudaEventRecord(B->ev_fork, st));
+  bool joined[8] = {};
+  for (int k = kNumClasses; k >= 0; --k) {
+    const int count = taken(k);
+    if (!count) continue;
+    cudaStream_t q = B->fork[k];
+    SK_CUDA(cudaStreamWaitEvent(q, B->ev_fork, 0));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    if (k == kNumClasses) {
+      BatchView rest = bv;
+      rest.order = B->cl_order + B->cl_first[static_cast<size_t>(k)];
+      rest.nsys = count;
+      BatchArgs ra = a;
+      ra.counter = B->counter + k;
+      ra.limit = count;
+      v.fn<<<std::min(ctas, count), v.NT, 0, q>>>(rest, ra);
+    } else {
+      const ClusterClass& c = kClasses[k];
+      ClusterView cv{B->sys_off, B->cl_order + B->cl_first[static_cast<size_t>(k)], count, B->cl_slice0, B->cl_off,
+                     B->cl_len, B->cl_col, B->cl_val, c.cap};
+      cudaLaunchConfig_t cfg{};
+      cudaLaunchAttribute attr[1];
+      cfg.gridDim = dim3(static_cast<unsigned>(std::min(B->cl_ctas[k], count * c.C)));
+      cfg.blockDim = dim3(static_cast<unsigned>(c.NT));
+      cfg.dynamicSmemBytes = c.smem();
+      cfg.stream = q;
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = static_cast<unsigned>(c.C);
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      SK_CUDA(cudaLaunchKernelEx(&cfg, c.fn, cv, a, B->counter + k));
+    }
+    SK_CUDA(cudaEventRecord(B->ev_join[k], q));
+    joined[k] = true;
+  }
+  for (int k = 0; k <= kNumClasses; ++k)
+    if (joined[k]) SK_CUDA(cudaStreamWaitEvent(st, B->ev_join[k], 0));
+  return SK_OK;
+}
+
+// Builds the sliced copy (from the CSR arrays on the device and the host row
+// pointers) of the systems that a class takes.  Without it (no such system,
+// too much padding, no memory) the batch runs on batched_cg_kernel.
+sk_status build_cluster_copy(sk_batch_s* B, const int64_t* sys_off, const int64_t* rp, const std::vector<int>& order) {
+  for (int k = 0; k < kNumClasses; ++k) B->cl_ctas[k] = cluster_ctas(kClasses[k]);
+  std::vector<int> cls(static_cast<size_t>(B->nsys), kNumClasses), slice0(static_cast<size_t>(B->nsys) + 1), off;
+  std::vector<std::vector<int>> of(kNumClasses + 1);
+  off.push_back(0);
+  i64 entries = 0;
+  for (i64 s = 0; s < B->nsys; ++s) {
+    const i64 a = sys_off[s], n = sys_off[s + 1] - a;
+    slice0[static_cast<size_t>(s)] = static_cast<int>(off.size()) - 1;
+    int k = class_of(n);
+    if (k < kNumClasses && B->cl_ctas[k] <= 0) k = kNumClasses;
+    if (k == kNumClasses) continue;
+    const size_t first = off.size();
+    i64 padded = 0;
+    bool fits = true;
+    for (i64 i = 0; i < n && fits; i += 32) {
+      i64 w = 0;
+      for (i64 l = i; l < std::min(n, i + 32); ++l) w = std::max(w, rp[a + l + 1] - rp[a + l]);
+      fits = w <= kClMaxLen;
+      padded += 32 * w;
+      off.push_back(static_cast<int>(entries + padded));
+    }
+    const i64 nnz = rp[a + n] - rp[a];
+    fits = fits && padded <= 2 * nnz + 1024 && entries + padded < (i64(1) << 31) - 64;
+    if (!fits) {
+      off.resize(first);
+      continue;
+    }
+    entries += padded;
+    cls[static_cast<size_t>(s)] = k;
+  }
+  slice0[static_cast<size_t>(B->nsys)] = static_cast<int>(off.size()) - 1;
+  const i64 slices = static_cast<i64>(off.size()) - 1;
+  if (slices == 0) return SK_OK;
+  B->cl_at.assign(kNumClasses + 1, {});
+  for (size_t q = 0; q < order.size(); ++q) {
+    const int k = cls[static_cast<size_t>(order[q])];
+    of[static_cast<size_t>(k)].push_back(order[q]);
+    B->cl_at[static_cast<size_t>(k)].push_back(static_cast<int>(q));
+  }
+  std::vector<int> flat;
+  for (auto const& l : of) {
+    B->cl_first.push_back(static_cast<int>(flat.size()));
+    flat.insert(flat.end(), l.begin(), l.end());
+  }
+  auto alloc = [&](size_t bytes, const void* src) -> void* {
+    void* m = nullptr;
+    if (cudaMalloc(&m, bytes + 64) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    B->allocs.push_back(m);
+    if (src && cudaMemcpy(m, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
+    return m;
+  };
+  B->cl_slice0 = static_cast<int*>(alloc(slice0.size() * 4, slice0.data()));
+  B->cl_off = static_cast<int*>(alloc(off.size() * 4, off.data()));
+  B->cl_order = static_cast<int*>(alloc(flat.size() * 4, flat.data()));
+  B->cl_len = static_cast<unsigned char*>(alloc(static_cast<size_t>(slices) * 32, nullptr));
+  B->cl_col = static_cast<unsigned short*>(alloc(static_cast<size_t>(entries) * 2, nullptr));
+  float* val = static_cast<float*>(alloc(static_cast<size_t>(entries) * 4, nullptr));
+  if (!B->cl_slice0 || !B->cl_off || !B->cl_order || !B->cl_len || !B->cl_col || !val) return SK_OK;
+  for (int k = 0; k <= kNumClasses; ++k) {
+    SK_CUDA(cudaStreamCreateWithFlags(&B->fork[k], cudaStreamNonBlocking));
+    SK_CUDA(cudaEventCreateWithFlags(&B->ev_join[k], cudaEventDisableTiming));
+  }
+  SK_CUDA(cudaEventCreateWithFlags(&B->ev_fork, cudaEventDisableTiming));
+  cl_fill_kernel<<<static_cast<unsigned>(B->nsys), 256, 0, B->stream>>>(view_of(B), B->cl_slice0, B->cl_off,
+                                                                        B->cl_len, B->cl_col, val);
+  SK_CUDA(cudaGetLastError());
+  SK_CUDA(cudaStreamSynchronize(B->stream));
+  B->cl_val = val;
+  return SK_OK;
 }
 
 }  // namespace
@@ -446,6 +949,11 @@ SK_API sk_status sk_batch_create(sk_batch* out, int64_t nsys, const int64_t* sys
   B->vals = static_cast<float*>(v);
   B->counter = static_cast<int*>(c);
   if (nnz) cudaMemcpy(v, values, nnz * 4, cudaMemcpyHostToDevice);
+  std::vector<int> queue(order.begin(), order.end());
+  if ((st = build_cluster_copy(B, sys_offsets, row_ptr, queue)) != SK_OK) {
+    sk_batch_destroy(B);
+    return st;
+  }
   *out = B;
   return SK_OK;
 }
@@ -456,6 +964,11 @@ SK_API sk_status sk_batch_destroy(sk_batch B) {
   if (B->graph) cudaGraphExecDestroy(B->graph);
   for (void* p : B->allocs) cudaFree(p);
   if (B->ws) cudaFree(B->ws);
+  for (cudaStream_t q : B->fork)
+    if (q) cudaStreamDestroy(q);
+  for (cudaEvent_t e : B->ev_join)
+    if (e) cudaEventDestroy(e);
+  if (B->ev_fork) cudaEventDestroy(B->ev_fork);
   if (B->stream) cudaStreamDestroy(B->stream);
   delete B;
   return SK_OK;
@@ -471,7 +984,7 @@ SK_API sk_status sk_batched_cg_solve(sk_batch B, const double* b_dev, double* x_
   SK_CHECK(vi >= 0, SK_INVALID_ARG, "lanes_per_row must be 1, 2, 4 or 8 and threads_per_cta 256, 512 or 1024");
   const Variant& v = kVariants[vi];
   const int ctas = ctas_for(B, v);
-  sk_status st = ensure_batch_ws(B, ctas);
+  sk_status st = ensure_batch_ws(B, v, ctas);
   if (st != SK_OK) return st;
   SK_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(s)));
   // The launch (queue reset + persistent kernel) is captured once into a
@@ -486,21 +999,23 @@ SK_API sk_status sk_batched_cg_solve(sk_batch B, const double* b_dev, double* x_
       B->graph = nullptr;
     }
     BatchArgs a = make_args(B, ctas, b_dev, x_dev, cfg, res, static_cast<int>(B->nsys));
-    BatchView bv = view_of(B);
     cudaGraph_t g = nullptr;
     SK_CUDA(cudaStreamBeginCapture(B->stream, cudaStreamCaptureModeThreadLocal));
-    cudaMemsetAsync(B->counter, 0, sizeof(int), B->stream);
-    v.fn<<<ctas, v.NT, 0, B->stream>>>(bv, a);
-    SK_CUDA(cudaStreamEndCapture(B->stream, &g));
-    cudaError_t e = cudaGraphInstantiate(&B->graph, g, 0);
-    cudaGraphDestroy(g);
-    if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
+    const i64 before = g_launches.load();
+    st = enqueue_batch(B, v, ctas, a, static_cast<int>(B->nsys));
+    B->graph_launches = g_launches.load() - before;
+    g_launches.fetch_sub(B->graph_launches);  // counted at each replay instead
+    cudaError_t e = cudaStreamEndCapture(B->stream, &g);
+    if (st == SK_OK && e == cudaSuccess) e = cudaGraphInstantiate(&B->graph, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (st != SK_OK) return st;
+    if (e != cudaSuccess) return cuda_fail(e, "batched solve capture");
     std::copy(key, key + 4, B->graph_key);
     B->graph_variant = vi;
     B->graph_ctas = ctas;
     B->graph_cfg = *cfg;
   }
-  g_launches.fetch_add(1, std::memory_order_relaxed);
+  g_launches.fetch_add(B->graph_launches, std::memory_order_relaxed);
   SK_CUDA(cudaGraphLaunch(B->graph, B->stream));
   SK_CUDA(cudaStreamSynchronize(B->stream));
   return SK_OK;
@@ -520,17 +1035,14 @@ SK_API sk_status sk_batched_autotune(sk_batch B, const double* b_dev, double* x_
   for (int i = 0; i < kNumVariants; ++i) {
     const Variant& v = kVariants[i];
     const int ctas = std::min(ctas_for(B, v), limit);
-    sk_status st = ensure_batch_ws(B, ctas_for(B, v));
+    sk_status st = ensure_batch_ws(B, v, ctas_for(B, v));
     if (st != SK_OK) return st;
     BatchArgs a = make_args(B, ctas, b_dev, x_dev, cfg, res, limit);
-    BatchView bv = view_of(B);
     float ms = 0.0f;
     for (int rep = 0; rep < 2; ++rep) {  // the first run warms the caches
-      SK_CUDA(cudaMemsetAsync(B->counter, 0, sizeof(int), B->stream));
       SK_CUDA(cudaMemsetAsync(x_dev, 0, B->nrow * sizeof(double), B->stream));
       SK_CUDA(cudaEventRecord(e0, B->stream));
-      g_launches.fetch_add(1, std::memory_order_relaxed);
-      v.fn<<<ctas, v.NT, 0, B->stream>>>(bv, a);
+      if ((st = enqueue_batch(B, v, ctas, a, limit)) != SK_OK) return st;
       SK_CUDA(cudaEventRecord(e1, B->stream));
       SK_CUDA(cudaEventSynchronize(e1));
       SK_CUDA(cudaEventElapsedTime(&ms, e0, e1));

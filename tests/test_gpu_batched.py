@@ -69,3 +69,54 @@ def test_batch_rejects_coupled_systems(gpu_lib):
     ci = np.array([0, 1, 2, 2, 3], np.int64)  # row 1 reaches column 2 of the second system
     with pytest.raises(_lib.SkError):
         gpu.Batch(offs, rp, ci, np.ones(5, np.float32))
+
+
+def test_cluster_classes_and_their_edges(gpu_lib):
+    """One lane per row solves a system on a cluster of 1 to 8 CTAs by its
+    size: systems at the classes' limits and one row beside them, with rows
+    and slices that do not fill, an empty one, one whose columns are spread
+    over the whole system (every gather crosses CTAs), and the two kinds that
+    stay with the general kernel (more than 65,536 rows, a row of more than
+    64 entries).  Each reaches the FP64 tolerance on its true residual."""
+    import scipy.sparse as sp
+    import torch
+    rng = np.random.default_rng(7)
+
+    def chain(n):
+        return sp.diags([np.full(n - 1, -1.0), np.full(n, 2.5), np.full(n - 1, -1.0)], [-1, 0, 1]) if n > 1 else \
+            sp.csr_matrix([[2.5]])
+
+    mats = [chain(n) for n in (1, 31, 32, 33, 1000, 5376, 5377, 10848, 10849, 21696, 21697, 43392, 43393, 65536,
+                               65537)]
+    g = matgen.laplacian_2d_dirichlet(171)
+    L = sp.csr_matrix((g.values(), g.col_ind(), g.row_ptr()), g.shape()) + 0.1 * sp.identity(171 * 171)
+    perm = rng.permutation(171 * 171)
+    mats.append(L.tocsr()[perm][:, perm])
+    arrow = sp.identity(300).tolil()
+    arrow[0, :70] = 0.01
+    arrow[:70, 0] = 0.01
+    arrow[0, 0] = 2.0
+    mats += [arrow, sp.csr_matrix((0, 0)), chain(17)]
+    offs, rps, cols, vals, nnz = [0], [], [], [], 0
+    for m in mats:
+        m = sp.csr_matrix(m).astype(np.float32)
+        m.sort_indices()
+        rps.append(m.indptr[:-1].astype(np.int64) + nnz)
+        cols.append(m.indices.astype(np.int64) + offs[-1])
+        vals.append(m.data)
+        nnz += m.nnz
+        offs.append(offs[-1] + m.shape[0])
+    rp = np.concatenate(rps + [[nnz]])
+    ci, va = np.concatenate(cols), np.concatenate(vals)
+    B = gpu.Batch(np.array(offs), rp, ci, va)
+    b = rng.uniform(-1, 1, offs[-1])
+    bd = torch.from_numpy(b).cuda()
+    full = sp.csr_matrix((va.astype(np.float64), ci, rp), (offs[-1], offs[-1]))
+    for threads in (512, 1024):
+        xd = torch.zeros_like(bd)
+        _, _, rel, conv = B.solve(bd, xd, gpu.Batch_config(threads_per_cta=threads))
+        assert conv.all() and (rel < 1e-10).all()
+        r = b - full @ xd.cpu().numpy()
+        for s in range(len(mats)):
+            a, e = offs[s], offs[s + 1]
+            assert np.linalg.norm(r[a:e]) <= 1.0001e-10 * np.linalg.norm(b[a:e]), (s, e - a)
