@@ -215,9 +215,12 @@ SK_API sk_status sk_matrix_info(sk_matrix A, int64_t info[8]);
  *   SK_LAYOUT_SPLIT     CSR split by row length (skewed rows);
  *   SK_LAYOUT_PANELS    CSR column panels (sk_matrix_add_panels: x staged
  *                       panel by panel in shared memory, every row summed
- *                       in column order). */
+ *                       in column order);
+ *   SK_LAYOUT_STENCIL   stencil copy (built for large square CSR handles on 5
+ *                       or 7 diagonals; half of them when the matrix is
+ *                       symmetric bit for bit). */
 enum { SK_LAYOUT_NATIVE = 0, SK_LAYOUT_SELL = 1, SK_LAYOUT_DIAGONALS = 2, SK_LAYOUT_SPLIT = 3,
-       SK_LAYOUT_PANELS = 4 };
+       SK_LAYOUT_PANELS = 4, SK_LAYOUT_STENCIL = 5 };
 SK_API sk_status sk_matrix_layout(sk_matrix A, int32_t* layout);
 
 /* Adds an FP32 copy of the values of an FP64 CSR handle (indices shared),

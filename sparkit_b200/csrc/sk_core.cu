@@ -416,7 +416,9 @@ sk_status csr_finish(sk_matrix A, const int64_t* row_ptr, cudaStream_t st_) {
   if ((st = upload_vector(A, tiles, &A->csr.tiles, st_)) != SK_OK) return st;
   if ((st = upload_vector(A, lanes, &A->csr.lanes, st_)) != SK_OK) return st;
   if ((st = build_sell(A, row_ptr, st_)) != SK_OK) return st;
-  return A->csr.sell ? SK_OK : build_hybrid(A, row_ptr, st_);
+  if (!A->csr.sell) return build_hybrid(A, row_ptr, st_);
+  SK_CUDA(cudaStreamSynchronize(st_));
+  return build_stencil(A);
 }
 
 }  // namespace sk
@@ -740,7 +742,8 @@ sk_status sk_matrix_layout(sk_matrix A, int32_t* layout) {
   *layout = SK_LAYOUT_NATIVE;
   if (A->format == SK_CSR) {
     const auto& C = A->csr;
-    *layout = C.dia_n ? SK_LAYOUT_DIAGONALS
+    *layout = C.st_n ? SK_LAYOUT_STENCIL
+              : C.dia_n ? SK_LAYOUT_DIAGONALS
               : C.sell ? SK_LAYOUT_SELL
               : C.panel ? SK_LAYOUT_PANELS
               : C.hyb ? SK_LAYOUT_SPLIT

@@ -93,6 +93,48 @@ __global__ void dia_fill_kernel(i64 n, const int* __restrict__ rp, const int* __
   }
 }
 
+// bad = 1 unless every entry (r, c), c != r, meets an entry (c, r) of the same
+// bits.
+template <typename T>
+__global__ void stencil_symmetric_kernel(i64 n, const int* __restrict__ rp, const int* __restrict__ ci,
+                                         const T* __restrict__ va, int* bad) {
+  for (i64 r = blockIdx.x * static_cast<i64>(blockDim.x) + threadIdx.x; r < n;
+       r += static_cast<i64>(gridDim.x) * blockDim.x) {
+    for (int k = rp[r]; k < rp[r + 1]; ++k) {
+      const int c = ci[k];
+      bool found = false;
+      for (int q = rp[c]; q < rp[c + 1] && !found; ++q)
+        if (ci[q] == static_cast<int>(r)) {
+          if constexpr (sizeof(T) == 8)
+            found = __double_as_longlong(va[q]) == __double_as_longlong(va[k]);
+          else
+            found = __float_as_int(va[q]) == __float_as_int(va[k]);
+        }
+      if (!found) *bad = 1;
+    }
+  }
+}
+
+// The planes of the diagonals first .. o.n - 1 and every row's mask of all.
+template <typename T>
+__global__ void stencil_fill_kernel(i64 n, const int* __restrict__ rp, const int* __restrict__ ci,
+                                    const T* __restrict__ va, Offsets o, int first, T* __restrict__ planes,
+                                    unsigned short* __restrict__ mask) {
+  const int np = o.n - first;
+  for (i64 r = blockIdx.x * static_cast<i64>(blockDim.x) + threadIdx.x; r < n;
+       r += static_cast<i64>(gridDim.x) * blockDim.x) {
+    unsigned m = 0;
+    for (int k = rp[r]; k < rp[r + 1]; ++k) {
+      const int off = ci[k] - static_cast<int>(r);
+      int d = 0;
+      while (d + 1 < o.n && o.off[d] != off) ++d;  // every offset is in the set
+      if (d >= first) planes[((r >> 5) * np + d - first) * 32 + (r & 31)] = va[k];
+      m |= 1u << d;
+    }
+    mask[r] = static_cast<unsigned short>(m);
+  }
+}
+
 __global__ void dia_to_float_kernel(const double* __restrict__ in, float* __restrict__ out, i64 n) {
   for (i64 i = blockIdx.x * static_cast<i64>(blockDim.x) + threadIdx.x; i < n;
        i += static_cast<i64>(gridDim.x) * blockDim.x)
@@ -132,6 +174,68 @@ sk_status dia_pattern(sk_matrix A, std::vector<int>* offsets) {
   const i64 nd = static_cast<i64>(offs.size());
   if (nd == 0 || nd * n > 2 * A->nnz) return SK_OK;  // planes more than half empty
   *offsets = offs;
+  return SK_OK;
+}
+
+sk_status csr_symmetric(sk_matrix A, std::vector<int> const& offs, bool* sym) {
+  *sym = false;
+  const size_t nd = offs.size();
+  if (A->nrow != A->ncol) return SK_OK;
+  for (size_t d = 0; d < nd; ++d)
+    if (offs[d] != -offs[nd - 1 - d]) return SK_OK;
+  int* bad = nullptr;
+  int h = 0;
+  SK_CUDA(cudaMalloc(&bad, sizeof(int)));
+  cudaError_t e = cudaMemsetAsync(bad, 0, sizeof(int), A->stream);
+  if (A->dtype == SK_F64)
+    SK_LAUNCH(stencil_symmetric_kernel<double>, grid_for(A->nrow), kThreads, 0, A->stream, A->nrow, A->csr.row_ptr,
+              A->csr.col_ind, static_cast<const double*>(A->csr.vals), bad);
+  else
+    SK_LAUNCH(stencil_symmetric_kernel<float>, grid_for(A->nrow), kThreads, 0, A->stream, A->nrow, A->csr.row_ptr,
+              A->csr.col_ind, static_cast<const float*>(A->csr.vals), bad);
+  if (e == cudaSuccess) e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&h, bad, sizeof(int), cudaMemcpyDeviceToHost, A->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(A->stream);
+  cudaFree(bad);
+  if (e != cudaSuccess) return cuda_fail(e, "symmetry check");
+  *sym = h == 0;
+  return SK_OK;
+}
+
+sk_status build_stencil(sk_matrix A) {
+  const i64 n = A->nrow;
+  if (A->format != SK_CSR || n != A->ncol || A->nnz < kStencilMinEntries) return SK_OK;
+  std::vector<int> offs;
+  sk_status s = dia_pattern(A, &offs);
+  if (s != SK_OK) return s;
+  const int nd = static_cast<int>(offs.size());
+  if ((nd != 5 && nd != 7) || n * nd >= (i64(1) << 31) - 64) return SK_OK;
+  bool sym = false;
+  if ((s = csr_symmetric(A, offs, &sym)) != SK_OK) return s;
+  const int first = sym ? nd / 2 : 0;
+  const i64 len = (n + 31) / 32 * 32 * (nd - first);
+  const size_t V = vbytes(A->dtype);
+  void *planes = nullptr, *mask = nullptr;
+  if ((s = dev_alloc(A, &planes, len * V + 64)) != SK_OK) return s;
+  if ((s = dev_alloc(A, &mask, (n + 64) * 2)) != SK_OK) return s;
+  SK_CUDA(cudaMemsetAsync(planes, 0, len * V + 64, A->stream));
+  Offsets o{};
+  o.n = nd;
+  for (int d = 0; d < nd; ++d) o.off[d] = A->csr.st_off[d] = offs[static_cast<size_t>(d)];
+  if (A->dtype == SK_F64)
+    SK_LAUNCH(stencil_fill_kernel<double>, grid_for(n), kThreads, 0, A->stream, n, A->csr.row_ptr, A->csr.col_ind,
+              static_cast<const double*>(A->csr.vals), o, first, static_cast<double*>(planes),
+              static_cast<unsigned short*>(mask));
+  else
+    SK_LAUNCH(stencil_fill_kernel<float>, grid_for(n), kThreads, 0, A->stream, n, A->csr.row_ptr, A->csr.col_ind,
+              static_cast<const float*>(A->csr.vals), o, first, static_cast<float*>(planes),
+              static_cast<unsigned short*>(mask));
+  SK_CUDA(cudaGetLastError());
+  SK_CUDA(cudaStreamSynchronize(A->stream));
+  A->csr.st_vals = planes;
+  A->csr.st_mask = static_cast<unsigned short*>(mask);
+  A->csr.st_sym = sym;
+  A->csr.st_n = nd;
   return SK_OK;
 }
 

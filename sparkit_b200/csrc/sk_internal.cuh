@@ -24,6 +24,9 @@ constexpr int kTileNnz = 2048;   // CSR: stored entries staged per CTA
 constexpr int kRowsMax = 256;    // CSR: rows per CTA (one per thread)
 constexpr int kBsrTileVals = 4096;  // BSR: block values staged per CTA
 constexpr int kMaxRed = 4;       // fused reductions carried per kernel
+constexpr i64 kStencilMinEntries = 1 << 19;  // below, the products are bound by launch latency
+constexpr i64 kTileSmem = 192 * 1024;    // bytes of x in a CTA's shared memory
+constexpr i64 kTileMinEntries = 1 << 20;  // fewest entries of the long rows
 constexpr int kSellMaxRow = 64;  // CSR rows up to this length use SELL-32
 constexpr int kDiaMax = 16;      // diagonals of the diagonal copy of a CSR handle
 constexpr int kPanelSmem = 220 * 1024;  // dynamic shared memory of a column-panel CTA (at most)
@@ -156,6 +159,16 @@ struct Csr {
   void* dia_vals = nullptr;
   float* dia_vals32 = nullptr;
   unsigned short* dia_mask = nullptr;
+  // Stencil copy (built at upload, sk_dia.cu) of a square handle of at least
+  // kStencilMinEntries entries on 5 or 7 diagonals whose rows ascend: laid out
+  // like the diagonal copy.  Of a matrix that is symmetric bit for bit
+  // (st_sym) only the diagonals c >= r are stored, and A(r, r - o) is read
+  // where A(r - o, r) stands.
+  int st_n = 0;
+  bool st_sym = false;
+  int st_off[kDiaMax] = {};
+  void* st_vals = nullptr;
+  unsigned short* st_mask = nullptr;
   // Symmetrically scaled FP32 copies for the Jacobi inner solve of the
   // mixed solver (sk_mixed.cu): S = D^-1/2 A D^-1/2 without its unit
   // diagonal, in the SELL-32 layout (sym_off, sym_len, sym_col, sym_val) or
@@ -401,6 +414,14 @@ sk_status build_dia_f32(sk_matrix A);
 // The column-panel copy of a CSR handle (host row pointers); a no-op when
 // the handle does not qualify (sk_matrix_add_panels).
 sk_status build_panel(sk_matrix A, const int64_t* rp, cudaStream_t st);
+// The panel-major copy of the long rows of a split handle; a no-op when it
+// does not qualify.
+sk_status build_tiles(sk_matrix A, i64 long_nnz, cudaStream_t st);
+void destroy_tiles(sk_matrix A);
+// Whether a square CSR handle on these diagonals is symmetric bit for bit.
+sk_status csr_symmetric(sk_matrix A, std::vector<int> const& offsets, bool* sym);
+// The stencil copy of a CSR handle; a no-op when it does not qualify.
+sk_status build_stencil(sk_matrix A);
 // The sorted diagonal offsets c - r of a CSR handle whose pattern fits the
 // diagonal copy (at most kDiaMax diagonals, columns ascending in every row,
 // planes at most half empty); empty when it does not.

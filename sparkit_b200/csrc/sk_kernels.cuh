@@ -772,6 +772,61 @@ dia_spmv_kernel(DiaArgs g, const T* __restrict__ va, const T* __restrict__ x, Ep
 }
 
 // ------------------------------------------------------------------
+// CSR through its stencil copy: one thread per row, all ND values and ND
+// entries of x issued before any is waited for; otherwise as dia_spmv_kernel
+// (absent diagonals read a clamped place and are left out by the mask, the
+// entries are added in ascending column order: the bits of the CSR row).
+//
+// What bounds a stencil product is the matrix stream.  SYM: the matrix is
+// symmetric bit for bit, only its upper diagonals are stored, and A(r, r - o)
+// is read at row r - o, which an earlier or neighbouring CTA has just brought
+// into L2: HBM carries 4 of 7 diagonals (FP64: 34 + 16 B a row against SELL's
+// 84 + 16).  The count is a template argument because the loads are what
+// hides the latency: with a run-time count in groups of 2 the same bytes took
+// 31 us at 128^3.  Back to back on the 7-point 128^3 Laplacian: FP64 34.8 us
+// through SELL, 26.2 through the diagonal copy, 19.3 here; FP32 12.4 (diagonal
+// copy 20.9).  64^3, in L2: FP64 4.2 us against 5.5.
+// ------------------------------------------------------------------
+struct StencilArgs {
+  int n;
+  const unsigned short* mask;
+  int off[7];
+};
+
+template <typename T, class Epi, int ND, bool SYM>
+__global__ void __launch_bounds__(kThreads, 4)
+stencil_spmv_kernel(StencilArgs g, const T* __restrict__ va, const T* __restrict__ x, Epi epi, RedWs ws,
+                    const Scalars* sc) {
+  constexpr int NR = Epi::kNR;
+  constexpr int NL = SYM ? ND / 2 : 0, NP = ND - NL;  // diagonals read at another row, planes stored
+  if (solve_done(sc)) return;
+  double red[NR > 0 ? NR : 1];
+#pragma unroll
+  for (int j = 0; j < (NR > 0 ? NR : 1); ++j) red[j] = 0.0;
+  for (int i = blockIdx.x * kThreads + threadIdx.x; i < g.n; i += gridDim.x * kThreads) {
+    const unsigned m = __ldcs(g.mask + i);
+    T v[ND], xv[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      const int c = min(max(i + g.off[d], 0), g.n - 1);
+      const int row = d < NL ? c : i;
+      const int p = d < NL ? ND - 1 - d - NL : d - NL;
+      const T* at = va + ((row >> 5) * NP + p) * 32 + (row & 31);
+      v[d] = SYM ? __ldg(at) : __ldcs(at);
+      xv[d] = __ldg(x + c);
+    }
+    T sum = T(0);
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+      if ((m >> d) & 1u) sum = add(sum, mul(v[d], xv[d]));
+    reduce_terms<NR>(ws, i, red, [&](double* rr) { epi(i, sum, rr); });
+  }
+  if constexpr (NR > 0) {
+    grid_reduce<NR>(red, ws, [&](const double* t) { epi.finalize(t); });
+  }
+}
+
+// ------------------------------------------------------------------
 // ELLPACK (slot-major): one thread per row, sequential over its slots,
 // stopping at the row's length (the reference stops at the first -1).
 // ------------------------------------------------------------------
@@ -1024,6 +1079,22 @@ void launch_spmv(const sk_matrix_s* A, const T* x, Epi const& epi, RedWs ws,
   if (A->nrow == 0) return;
   switch (A->format) {
     case SK_CSR: {
+      if (A->csr.st_n && !vals_override) {
+        const auto& C = A->csr;
+        StencilArgs g{static_cast<int>(A->nrow), C.st_mask, {}};
+        for (int d = 0; d < C.st_n; ++d) g.off[d] = C.st_off[d];
+        const T* v = static_cast<const T*>(C.st_vals);
+        const int grid = row_grid<Epi>(A, A->nrow, 4);
+        if (C.st_n == 7 && C.st_sym)
+          SK_LAUNCH((stencil_spmv_kernel<T, Epi, 7, true>), grid, kThreads, 0, st, g, v, x, epi, ws, sc);
+        else if (C.st_n == 7)
+          SK_LAUNCH((stencil_spmv_kernel<T, Epi, 7, false>), grid, kThreads, 0, st, g, v, x, epi, ws, sc);
+        else if (C.st_sym)
+          SK_LAUNCH((stencil_spmv_kernel<T, Epi, 5, true>), grid, kThreads, 0, st, g, v, x, epi, ws, sc);
+        else
+          SK_LAUNCH((stencil_spmv_kernel<T, Epi, 5, false>), grid, kThreads, 0, st, g, v, x, epi, ws, sc);
+        break;
+      }
       if (A->csr.dia_n) {
         const T* v = vals_override ? vals_override : static_cast<const T*>(A->csr.dia_vals);
         SK_LAUNCH((dia_spmv_kernel<T, Epi, SpmvTune<T, Epi>::kDiaMinB>),

@@ -180,7 +180,7 @@ class Device_matrix:
         keys = ("format", "dtype", "nrow", "ncol", "nnz", "width", "device_bytes", "spmv_bytes")
         return dict(zip(keys, list(arr)))
 
-    LAYOUTS = ("native", "sell", "diagonals", "split", "panels")
+    LAYOUTS = ("native", "sell", "diagonals", "split", "panels", "stencil")
 
     def layout(self):
         """The device layout the product runs on (sk_matrix_layout): one of
