@@ -285,11 +285,12 @@ static sk_status build_sell(sk_matrix A, const int64_t* rp, cudaStream_t st_) {
   if (n == 0 || A->nnz == 0) return SK_OK;
   const i64 nslices = (n + 31) / 32;
   std::vector<int> off(static_cast<size_t>(nslices) + 1, 0);
-  i64 total = 0;
+  i64 total = 0, widest = 0;
   for (i64 s = 0; s < nslices; ++s) {
     i64 w = 0;
     for (i64 i = 32 * s; i < std::min(n, 32 * s + 32); ++i) w = std::max<i64>(w, rp[i + 1] - rp[i]);
     if (w > kSellMaxRow) return SK_OK;
+    widest = std::max(widest, w);
     off[static_cast<size_t>(s)] = static_cast<int>(total);
     total += 32 * w;
     if (total > (i64(1) << 31) - 64) return SK_OK;
@@ -309,6 +310,7 @@ static sk_status build_sell(sk_matrix A, const int64_t* rp, cudaStream_t st_) {
   A->csr.sell_vals = val;
   A->csr.sell_len = static_cast<unsigned char*>(len);
   A->csr.sell_entries = total;
+  A->csr.sell_width = static_cast<int>(widest);
   if (A->dtype == SK_F64)
     SK_LAUNCH(csr_to_sell_kernel<double>, ceil_div(n, kThreads), kThreads, 0, st_, n, A->csr.row_ptr,
               A->csr.col_ind, static_cast<const double*>(A->csr.vals), A->csr.sell_off, A->csr.sell_col,

@@ -103,6 +103,7 @@ struct Csr {
   int* sell_off = nullptr;             // nslices + 1 entry offsets
   unsigned char* sell_len = nullptr;   // entries per row
   i64 sell_entries = 0;                // padded size
+  int sell_width = 0;                  // entries of the longest row
   // Split product for skewed rows (when SELL-32 is refused and rows longer
   // than kHybLong entries hold most of the entries): the long rows, by
   // decreasing length, one warp each; the short rows, in row order, one

@@ -47,11 +47,11 @@ constexpr int kPT = 512;   // threads per CTA (SELL: one CTA per SM, up to 128 r
                            // diagonal copy: two CTAs per SM, up to 64)
 constexpr int kPW = kPT / 32;
 constexpr int kPU = 8;     // SELL slots loaded together
-constexpr int kSlot = 4;   // doubles per CTA and reduction
+constexpr int kSlot = 3;   // most sums of one reduction
 
 struct SyncWords {
   unsigned long long arrived;  // total arrivals, never reset during a solve
-  int err;
+  int err;                     // a wait ran out
   int converged;
   long long iterations;
   double rnorm;
@@ -72,7 +72,7 @@ struct PArgs {
   float* d;
   float* p;
   float* q;
-  double* slots;  // [2][grid][kSlot]
+  double* slots;  // [2][kSlot][CTA]
   SyncWords* sync;
   float tol;
   long long max_iters;
@@ -97,89 +97,116 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// Grid barrier on one monotonic arrival counter: barrier number e (from 1)
-// is passed when the counter reaches e * gridDim.x (+ bias, which only the
-// timeout tests set).  False: a wait ran out (here or in another CTA) and
-// the kernel must return.  The clock and the error word are read once per
-// 256 polls.
-__device__ bool grid_barrier(SyncWords* s, unsigned& epoch, unsigned long long wait_ns, unsigned bias) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    epoch += 1;
-    const unsigned long long target = static_cast<unsigned long long>(epoch) * gridDim.x + bias;
-    arrive_release(&s->arrived);
-    unsigned long long t0 = 0;
-    for (unsigned spins = 0; ld_acquire(&s->arrived) < target; ++spins) {
-      if ((spins & 255u) == 255u) {
-        if (*reinterpret_cast<volatile int*>(&s->err) != 0) {
-          ok = 0;
-          break;
-        }
-        const unsigned long long t = global_ns();
-        if (t0 == 0) {
-          t0 = t;
-        } else if (t - t0 > wait_ns) {
-          atomicExch(&s->err, 1);
-          ok = 0;
-          break;
-        }
+// Waits (one thread) until `target` arrivals were counted.  False: the wait
+// ran out here or in another CTA.  The clock and the error word are read once
+// per 256 polls.
+__device__ __forceinline__ bool wait_arrivals(SyncWords* s, unsigned long long target, unsigned long long wait_ns) {
+  unsigned long long t0 = 0;
+  for (unsigned spins = 0; ld_acquire(&s->arrived) < target; ++spins) {
+    if ((spins & 255u) == 255u) {
+      if (*reinterpret_cast<volatile int*>(&s->err) != 0) return false;
+      const unsigned long long t = global_ns();
+      if (t0 == 0) {
+        t0 = t;
+      } else if (t - t0 > wait_ns) {
+        atomicExch(&s->err, 1);
+        return false;
       }
     }
-    s_ok = ok;
   }
-  __syncthreads();
-  return s_ok != 0;
+  return true;
 }
 
 // Sums v over the grid into every thread of every CTA (the same bits
-// everywhere): block tree, then CTA slots summed in CTA order by warp 0.
-// Consecutive reductions alternate between the two slot sets.
-template <int NR>
-__device__ __forceinline__ bool grid_allreduce(double (&v)[NR], PArgs const& a, int set, unsigned& epoch) {
+// everywhere) and makes every vector entry written before visible after it:
+// a block tree, one slot per CTA and value, an arrival on one monotonic counter
+// (exchange number e, from 1, is complete at e * gridDim.x arrivals, + bias,
+// which only the timeout tests set), then the slots in CTA order.  Between
+// the two block barriers warp 0 alone does all of it, so that no step waits on
+// a third.  Consecutive sums alternate between two slot sets.  False: a wait
+// ran out and the kernel must return.
+//
+// Measured alone (148 CTAs of 512 threads): 1.87 us, against 2.08 with two
+// more block barriers.  Values that carry their own arrival to a mailbox of
+// every CTA (no counter, no fence) took 2.97 us, through one summing CTA 2.58,
+// through clusters of 2 to 16 CTAs 2.9 to 3.3.
+//
+// WIDE: two CTAs per SM, whose slots are too many for one warp to read in one
+// round trip: a thread each, after a third barrier.
+template <int NR, bool WIDE = false>
+__device__ __forceinline__ bool grid_allreduce(double (&v)[NR], PArgs const& a, unsigned& epoch) {
   __shared__ double s_part[kPW][kSlot];
   __shared__ double s_tot[kSlot];
+  __shared__ int s_ok;
+  constexpr int U = 5;  // slots a lane reads together
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, grid = static_cast<int>(gridDim.x);
   warp_reduce<NR>(v);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (lane == 0)
 #pragma unroll
     for (int j = 0; j < NR; ++j) s_part[warp][j] = v[j];
+  epoch += 1;
   __syncthreads();
-  double* slot = a.slots + static_cast<size_t>(set) * gridDim.x * kSlot;
   if (warp == 0) {
     double t[NR];
 #pragma unroll
     for (int j = 0; j < NR; ++j) t[j] = lane < kPW ? s_part[lane][j] : 0.0;
     warp_reduce<NR>(t);
-    if (lane == 0)
+    double* slot = a.slots + static_cast<size_t>(epoch & 1) * kSlot * grid;
+    int ok = 1;
+    if (lane == 0) {
 #pragma unroll
-      for (int j = 0; j < NR; ++j) slot[static_cast<size_t>(blockIdx.x) * kSlot + j] = t[j];
+      for (int j = 0; j < NR; ++j) __stcg(slot + j * grid + blockIdx.x, t[j]);
+      arrive_release(&a.sync->arrived);
+      ok = wait_arrivals(a.sync, static_cast<unsigned long long>(epoch) * grid + a.bias, a.wait_ns);
+    }
+    if constexpr (!WIDE) {
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < NR; ++j) t[j] = 0.0;
+      for (int c0 = lane; c0 < grid; c0 += 32 * U) {
+        double x[NR][U];
+#pragma unroll
+        for (int j = 0; j < NR; ++j)
+#pragma unroll
+          for (int u = 0; u < U; ++u) x[j][u] = c0 + 32 * u < grid ? __ldcg(slot + j * grid + c0 + 32 * u) : 0.0;
+#pragma unroll
+        for (int j = 0; j < NR; ++j)
+#pragma unroll
+          for (int u = 0; u < U; ++u) t[j] += x[j][u];
+      }
+      warp_reduce<NR>(t);
+      if (lane == 0)
+#pragma unroll
+        for (int j = 0; j < NR; ++j) s_tot[j] = t[j];
+    }
+    if (lane == 0) s_ok = ok;
   }
-  if (!grid_barrier(a.sync, epoch, a.wait_ns, a.bias)) return false;
-  // every thread below gridDim.x reads one CTA's slot (one round trip),
-  // then a fixed tree over the CTA
-  double t[NR];
-#pragma unroll
-  for (int j = 0; j < NR; ++j)
-    t[j] = threadIdx.x < gridDim.x ? __ldcg(slot + static_cast<size_t>(threadIdx.x) * kSlot + j) : 0.0;
-  warp_reduce<NR>(t);
-  if (lane == 0)
-#pragma unroll
-    for (int j = 0; j < NR; ++j) s_part[warp][j] = t[j];
   __syncthreads();
-  if (warp == 0) {
+  if constexpr (WIDE) {
+    const int nw = (grid + 31) >> 5;
+    if (warp < nw) {
+      const double* slot = a.slots + static_cast<size_t>(epoch & 1) * kSlot * grid;
+      double t[NR];
 #pragma unroll
-    for (int j = 0; j < NR; ++j) t[j] = lane < kPW ? s_part[lane][j] : 0.0;
-    warp_reduce<NR>(t);
-    if (lane == 0)
+      for (int j = 0; j < NR; ++j)
+        t[j] = static_cast<int>(threadIdx.x) < grid ? __ldcg(slot + j * grid + threadIdx.x) : 0.0;
+      warp_reduce<NR>(t);
+      if (lane == 0)
 #pragma unroll
-      for (int j = 0; j < NR; ++j) s_tot[j] = t[j];
+        for (int j = 0; j < NR; ++j) s_part[warp][j] = t[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < NR; ++j) {
+      v[j] = s_part[0][j];
+      for (int w = 1; w < nw; ++w) v[j] += s_part[w][j];
+    }
+    __syncthreads();  // the parts are read before the next sum writes them
+  } else {
+#pragma unroll
+    for (int j = 0; j < NR; ++j) v[j] = s_tot[j];
   }
-  __syncthreads();
-#pragma unroll
-  for (int j = 0; j < NR; ++j) v[j] = s_tot[j];
-  return true;
+  return s_ok != 0;
 }
 
 // Row i's SELL position: its length and the offset of its slot 0.
@@ -397,7 +424,7 @@ __global__ void __launch_bounds__(kPT, DIA ? 2 : 1) inner_cg_kernel(PArgs a) {
     v0[0] += static_cast<double>(rr);
     v0[1] += static_cast<double>(UNIT ? mul(a.wdiag[i], rr) : rr);
   }
-  if (!grid_allreduce<2>(v0, a, 0, epoch)) return;
+  if (!grid_allreduce<2, DIA>(v0, a, epoch)) return;
   const float bnorm = sqrtf(static_cast<float>(v0[1]));
   float rho = static_cast<float>(v0[0]);
   float beta = 0.0f;
@@ -414,7 +441,7 @@ __global__ void __launch_bounds__(kPT, DIA ? 2 : 1) inner_cg_kernel(PArgs a) {
       if constexpr (DIA) pq[0] = phase_s_dia<UNIT, false>(a, t0, T, beta);
       else pq[0] = phase_s_sell<UNIT, false>(a, t0, T, beta);
     }
-    return grid_allreduce<1>(pq, a, 1, epoch);
+    return grid_allreduce<1, DIA>(pq, a, epoch);
   };
   double pq[1] = {0.0};
   if (!conv && a.max_iters > 0) {
@@ -464,7 +491,7 @@ __global__ void __launch_bounds__(kPT, DIA ? 2 : 1) inner_cg_kernel(PArgs a) {
         a.d[tail] = dn;
         a.r[tail] = rw;
       }
-      if (!grid_allreduce<2>(rr, a, 0, epoch)) return;
+      if (!grid_allreduce<2, DIA>(rr, a, epoch)) return;
       ++it;
       rn = sqrtf(static_cast<float>(UNIT ? rr[1] : rr[0]));
       conv = rn / bnorm < a.tol ? 1 : 0;
@@ -568,12 +595,11 @@ __global__ void __launch_bounds__(kPT, 1) cg64_kernel(Cg64Args a) {
     a.p0[i] = zi;
     v1[0] += mul(ri, zi);
   }
-  if (!grid_allreduce<1>(v1, a.g, 0, epoch)) return;
+  if (!grid_allreduce<1>(v1, a.g, epoch)) return;
   double rz = v1[0];
   long long it = 0;
   int conv = 0;
   double rn = 0.0, alpha = 0.0, beta = 0.0;
-  int set = 1;
   while (it < max_iters) {
     // 1: p (for k > 0), q = A p, <p, q>          (OpCgDirection, EpiCgPq)
     const double* pold = (it & 1) ? a.p0 : a.p1;  // step it - 1 wrote p[(it - 1) & 1]
@@ -599,8 +625,7 @@ __global__ void __launch_bounds__(kPT, 1) cg64_kernel(Cg64Args a) {
         pq[0] += mul(pi, qi);
       }
     }
-    if (!grid_allreduce<1>(pq, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<1>(pq, a.g, epoch)) return;
     alpha = rz / pq[0];
     // 2: x += alpha p, r -= alpha q, <r, r>, <r, D^-1 r>  (OpCgUpdate)
     double rr[2] = {0.0, 0.0};
@@ -611,8 +636,7 @@ __global__ void __launch_bounds__(kPT, 1) cg64_kernel(Cg64Args a) {
       rr[0] += mul(ri, ri);
       if (JAC) rr[1] += mul(ri, mul(invd[i], ri));
     }
-    if (!grid_allreduce<2>(rr, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<2>(rr, a.g, epoch)) return;
     ++it;
     rn = sqrt(rr[0]);
     if (a.hist && blockIdx.x == 0 && threadIdx.x == 0) a.hist[it - 1] = rn;
@@ -621,6 +645,163 @@ __global__ void __launch_bounds__(kPT, 1) cg64_kernel(Cg64Args a) {
     const double rz_new = JAC ? rr[1] : rr[0];
     beta = rz_new / rz;
     rz = rz_new;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->iters = it;
+    sc->converged = conv;
+    sc->done = 1;
+    sc->rnorm = rn;
+    sc->rz = rz;
+    sc->alpha = alpha;
+    sc->beta = beta;
+    sc->hist_len = a.hist ? it : 0;
+  }
+}
+
+// The same solve with everything but the neighbours' z and p on chip: a CTA's
+// slices of the matrix, z = D^-1 r and both halves of p of its rows in shared
+// memory, x, r, q and 1 / a_ii in the registers of the row's thread.  Where
+// cg64_kernel waits on L2 three times a step besides the two exchanges (its
+// matrix, its neighbours' entries, its vectors), this waits once, for the
+// entries of z and p in other CTAs' rows.  The same element arithmetic in the
+// same order: z_j is the product its neighbour would have formed.  256^2
+// Poisson, 718 steps: 4.99 ms through cg64_kernel, 3.89 so, of which the two
+// exchanges are 2.7.  (The same form of bi64_kernel, whose three phases gather
+// three vectors, was 8% slower than reading L2.)
+constexpr int kResRows = 4;  // rows of a thread
+
+struct Cg64Res {
+  int entries;  // matrix entries a CTA's shared memory holds
+  int per;      // rows of a CTA, a multiple of 32
+};
+
+template <bool JAC>
+__global__ void __launch_bounds__(kPT, 1) cg64_resident_kernel(Cg64Args a, Cg64Res m) {
+  extern __shared__ __align__(16) double res_smem[];
+  const int n = a.g.n, per = m.per;
+  double* s_val = res_smem;
+  double* s_z = s_val + m.entries;
+  double* s_p = s_z + per;  // two halves
+  int* s_col = reinterpret_cast<int*>(s_p + 2 * per);
+  unsigned epoch = 0;
+  const int r0 = min(n, static_cast<int>(blockIdx.x) * per), r1 = min(n, r0 + per);
+  const int lane = threadIdx.x & 31;
+  Scalars* sc = a.sc;
+  const double bnorm = sc->bnorm, tol = sc->tol;
+  const long long max_iters = sc->max_iters;
+  const double* x0 = a.x;
+  const int e0 = r0 < n ? __ldg(a.g.off + (r0 >> 5)) : 0;
+  const int e1 = r0 < n ? __ldg(a.g.off + ((r1 + 31) >> 5)) : 0;
+  for (int e = threadIdx.x; e < e1 - e0; e += kPT) {
+    s_val[e] = __ldg(a.val + e0 + e);
+    const int c = __ldg(a.g.col + e0 + e);
+    s_col[e] = c >= r0 && c < r1 ? c - r0 : ~c;  // a row of this CTA, or of another
+  }
+  double xr[kResRows], rr_[kResRows], qr[kResRows], dr[kResRows];
+  int len[kResRows], base[kResRows];
+  double* zg = a.r;  // the neighbours' view of z
+  // k = 0: r = b - A x, p = z = D^-1 r, rz = <r, z>   (EpiCgResid)
+  double v1[1] = {0.0};
+#pragma unroll
+  for (int u = 0; u < kResRows; ++u) {
+    const int l = threadIdx.x + u * kPT, i = r0 + l;
+    len[u] = base[u] = 0;
+    if (i < r1) {
+      len[u] = __ldg(a.g.len + i);
+      base[u] = __ldg(a.g.off + (i >> 5)) - e0 + lane;
+      const double ri = sub(a.b[i], sell_row64(a, i, [&](int j) { return x0[j]; }));
+      dr[u] = JAC ? a.invd[i] : 1.0;
+      const double zi = JAC ? mul(dr[u], ri) : ri;
+      rr_[u] = ri;
+      xr[u] = x0[i];
+      s_z[l] = zi;
+      s_p[l] = zi;
+      zg[i] = zi;
+      a.p0[i] = zi;
+      v1[0] += mul(ri, zi);
+    }
+  }
+  if (!grid_allreduce<1>(v1, a.g, epoch)) return;
+  double rz = v1[0];
+  long long it = 0;
+  int conv = 0;
+  double rn = 0.0, alpha = 0.0, beta = 0.0;
+  while (it < max_iters) {
+    // 1: p (for k > 0), q = A p, <p, q>          (OpCgDirection, EpiCgPq)
+    const int cur = static_cast<int>(it & 1);
+    const double* pold_g = cur ? a.p0 : a.p1;
+    double* pcur_g = cur ? a.p1 : a.p0;
+    double* s_new = s_p + cur * per;
+    const double* s_old = s_p + (cur ^ 1) * per;
+    const bool first = it == 0;
+    double pq[1] = {0.0};
+#pragma unroll
+    for (int u = 0; u < kResRows; ++u) {
+      const int l = threadIdx.x + u * kPT;
+      if (r0 + l >= r1) break;
+      double pi;
+      if (first) {
+        pi = s_new[l];  // written with z
+      } else {
+        pi = add(s_z[l], mul(beta, s_old[l]));
+        s_new[l] = pi;
+        pcur_g[r0 + l] = pi;
+      }
+      double sum = 0.0;
+      for (int k0 = 0; k0 < len[u]; k0 += 8) {
+        double zj[8], pj[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          if (k0 + k < len[u]) {
+            const int c = s_col[base[u] + 32 * (k0 + k)];
+            if (c >= 0) {
+              zj[k] = s_z[c];
+              pj[k] = s_old[c];
+            } else {
+              zj[k] = __ldcg(zg + ~c);
+              pj[k] = __ldcg(pold_g + ~c);
+            }
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+          if (k0 + k < len[u])
+            sum = add(sum, mul(s_val[base[u] + 32 * (k0 + k)], first ? zj[k] : add(zj[k], mul(beta, pj[k]))));
+      }
+      qr[u] = sum;
+      pq[0] += mul(pi, sum);
+    }
+    if (!grid_allreduce<1>(pq, a.g, epoch)) return;
+    alpha = rz / pq[0];
+    // 2: x += alpha p, r -= alpha q, <r, r>, <r, D^-1 r>  (OpCgUpdate)
+    double rr[2] = {0.0, 0.0};
+#pragma unroll
+    for (int u = 0; u < kResRows; ++u) {
+      const int l = threadIdx.x + u * kPT;
+      if (r0 + l >= r1) break;
+      xr[u] = add(mul(alpha, s_new[l]), xr[u]);
+      const double ri = sub(rr_[u], mul(alpha, qr[u]));
+      rr_[u] = ri;
+      const double zi = JAC ? mul(dr[u], ri) : ri;
+      s_z[l] = zi;
+      zg[r0 + l] = zi;
+      rr[0] += mul(ri, ri);
+      if (JAC) rr[1] += mul(ri, zi);
+    }
+    if (!grid_allreduce<2>(rr, a.g, epoch)) return;
+    ++it;
+    rn = sqrt(rr[0]);
+    if (a.hist && blockIdx.x == 0 && threadIdx.x == 0) a.hist[it - 1] = rn;
+    conv = rn / bnorm < tol ? 1 : 0;
+    if (conv || it >= max_iters) break;
+    const double rz_new = JAC ? rr[1] : rr[0];
+    beta = rz_new / rz;
+    rz = rz_new;
+  }
+#pragma unroll
+  for (int u = 0; u < kResRows; ++u) {
+    const int l = threadIdx.x + u * kPT;
+    if (r0 + l < r1) a.x[r0 + l] = xr[u];
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc->iters = it;
@@ -696,11 +877,10 @@ __global__ void __launch_bounds__(kPT, 1) bi64_kernel(Bi64Args a) {
     a.v[0][i] = 0.0;
     v1[0] += mul(ri, ri);
   }
-  if (!grid_allreduce<1>(v1, a.g, 0, epoch)) return;
+  if (!grid_allreduce<1>(v1, a.g, epoch)) return;
   double rho_new = v1[0], rho = 1.0, alpha = 1.0, omega = 1.0;
   long long iters = 0, hist_len = 0;
   int converged = 0, status = 0;
-  int set = 1;
   double last = 0.0;
   auto record = [&](double v) {
     if (a.hist && blockIdx.x == 0 && threadIdx.x == 0) a.hist[hist_len] = v;
@@ -732,8 +912,7 @@ __global__ void __launch_bounds__(kPT, 1) bi64_kernel(Bi64Args a) {
       vnew[i] = vi;
       rv[0] += mul(a.r_hat[i], vi);
     }
-    if (!grid_allreduce<1>(rv, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<1>(rv, a.g, epoch)) return;
     ++iters;
     if (rv[0] == 0.0) {
       status = SK_BREAKDOWN;
@@ -754,8 +933,7 @@ __global__ void __launch_bounds__(kPT, 1) bi64_kernel(Bi64Args a) {
       st[1] += mul(ti, ti);
       st[2] += mul(ti, si);
     }
-    if (!grid_allreduce<3>(st, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<3>(st, a.g, epoch)) return;
     const double sn = sqrt(st[0]);
     record(sn);
     if (sn / bnorm < tol) {  // half step converged: x += alpha p_hat (OpBiHalfOrS)
@@ -778,8 +956,7 @@ __global__ void __launch_bounds__(kPT, 1) bi64_kernel(Bi64Args a) {
         rr[1] += mul(a.r_hat[i], ri);
       }
     }
-    if (!grid_allreduce<2>(rr, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<2>(rr, a.g, epoch)) return;
     if (!skip) {
       rho = rho_new;
       const double rn = sqrt(rr[0]);
@@ -872,11 +1049,11 @@ __global__ void __launch_bounds__(kPT, 1) cgs64_kernel(Cgs64Args a) {
     a.u[i] = ri;
     v1[0] += mul(ri, ri);
   }
-  if (!grid_allreduce<1>(v1, a.g, 0, epoch)) return;
+  if (!grid_allreduce<1>(v1, a.g, epoch)) return;
   double rho = v1[0], alpha = 0.0, beta = 0.0, last = 0.0;
   long long iters = 0, hist_len = 0;
   int converged = 0, skip = 0;
-  int set = 1, cur = 0;
+  int cur = 0;
   bool upd = false;  // the previous step left a direction update to apply
   bool done = max_iters <= 0;
   while (!done) {
@@ -902,8 +1079,7 @@ __global__ void __launch_bounds__(kPT, 1) cgs64_kernel(Cgs64Args a) {
       a.q_hat[i] = qh;
       rq[0] += mul(a.r_hat[i], qh);
     }
-    if (!grid_allreduce<1>(rq, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<1>(rq, a.g, epoch)) return;
     if (up) cur ^= 1;
     alpha = rho / rq[0];
     // B: q, u_hat, x, r -= alpha A u_hat, ||r||^2, <r_hat, r>
@@ -927,8 +1103,7 @@ __global__ void __launch_bounds__(kPT, 1) cgs64_kernel(Cgs64Args a) {
       rr[0] += mul(ri, ri);
       rr[1] += mul(a.r_hat[i], ri);
     }
-    if (!grid_allreduce<2>(rr, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<2>(rr, a.g, epoch)) return;
     // EpiCgsR
     iters += 2;
     const double rn = sqrt(rr[0]);
@@ -1026,8 +1201,7 @@ __global__ void __launch_bounds__(kPT, 1) min64_kernel(Min64Args a) {
     a.dp[i] = 0.0;
     v1[0] += mul(vi, zi);
   }
-  if (!grid_allreduce<1>(v1, a.g, 0, epoch)) return;
-  int set = 1;
+  if (!grid_allreduce<1>(v1, a.g, epoch)) return;
   double beta = sqrt(v1[0]);
   double alpha = 0.0, eps = 0.0, delta = 0.0, rho = 0.0, phi = 0.0, phi_bar = beta;
   double cs_prev = 1.0, sn_prev = 0.0, cs = 1.0, sn = 0.0, cs_new = 0.0, sn_new = 0.0, inv_bn = 0.0;
@@ -1045,8 +1219,7 @@ __global__ void __launch_bounds__(kPT, 1) min64_kernel(Min64Args a) {
       a.z[i] = mul(a.z[i], inv_bn);
     }
     double none[1] = {0.0};  // the scaled z is gathered by the first product
-    if (!grid_allreduce<1>(none, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<1>(none, a.g, epoch)) return;
   }
   if (max_iters <= 0) done = true;
   bool pending = false, rotate = false;
@@ -1077,8 +1250,7 @@ __global__ void __launch_bounds__(kPT, 1) min64_kernel(Min64Args a) {
       a.w[i] = wi;
       zw[0] += mul(a.z[i], wi);
     }
-    if (!grid_allreduce<1>(zw, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<1>(zw, a.g, epoch)) return;
     pending = false;
     alpha = zw[0];
     // B: the Lanczos vector, q = M w, <w, q>
@@ -1090,8 +1262,7 @@ __global__ void __launch_bounds__(kPT, 1) min64_kernel(Min64Args a) {
       a.q[i] = qi;
       wq[0] += mul(wi, qi);
     }
-    if (!grid_allreduce<1>(wq, a.g, set, epoch)) return;
-    set ^= 1;
+    if (!grid_allreduce<1>(wq, a.g, epoch)) return;
     // min_step_finalize
     const double beta_new = sqrt(wq[0]);
     eps = mul(sn_prev, beta);
@@ -1380,8 +1551,8 @@ bool inner_persistent_ok(sk_matrix A, bool scaled) {
   return coop_grid(A, pick_kernel(use_dia(A, scaled), scaled)) > 0;
 }
 
-size_t inner_persistent_scratch(sk_matrix A) {
-  return sizeof(SyncWords) + static_cast<size_t>(2) * kPT * kSlot * sizeof(double) + 256;
+size_t inner_persistent_scratch(sk_matrix) {
+  return 256 + static_cast<size_t>(2) * kPT * kSlot * sizeof(double) + 256;
 }
 
 sk_status inner_cg_persistent(sk_matrix A, bool scaled, float* r, float* d, float* p, float* q, void* scratch,
@@ -1397,7 +1568,7 @@ sk_status inner_cg_persistent(sk_matrix A, bool scaled, float* r, float* d, floa
   const void* k = pick_kernel(dia, scaled);
   int grid = coop_grid(A, k);
   SK_CHECK(grid > 0, SK_NOT_SUPPORTED, "persistent inner solve does not fit on the device");
-  grid = std::min(grid, kPT);  // a CTA sums the grid's slots one per thread
+  grid = std::min(grid, kPT);  // the slots' size
   const int need = ceil_div(A->nrow, kPT);
   if (grid > need) grid = need;
   SyncWords* sync = static_cast<SyncWords*>(scratch);
@@ -1450,6 +1621,23 @@ sk_status inner_cg_persistent(sk_matrix A, bool scaled, float* r, float* d, floa
   return SK_OK;
 }
 
+// Dynamic shared memory of the resident kernels beside their 1.5 KB of
+// reduction scratch.
+constexpr size_t kResSmem = 224 * 1024;
+
+static bool resident_ok(sk_matrix A, const void* k) {
+  int optin = 0, per_sm = 0;
+  if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, A->device) != cudaSuccess ||
+      static_cast<size_t>(optin) < kResSmem + 2048 ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kResSmem)) !=
+          cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPT, kResSmem) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return per_sm > 0;
+}
+
 bool cg64_persistent_ok(sk_matrix A) {
   if (!A || A->format != SK_CSR || A->dtype != SK_F64 || !A->csr.sell || A->nrow <= 0) return false;
   if (A->nrow > kCg64MaxRows || summation_sequential()) return false;
@@ -1490,9 +1678,17 @@ sk_status cg64_persistent(sk_matrix A, const double* b, double* x, double* r, do
   a.invd = invd;
   a.hist = hist;
   a.sc = sc;
-  void* params[] = {&a};
+  // on chip when every CTA's slices and vectors fit its shared memory
+  Cg64Res m{};
+  m.per = ((a.g.n + grid - 1) / grid + 31) & ~31;
+  m.entries = m.per * C.sell_width;
+  const size_t smem = static_cast<size_t>(m.entries) * 12 + static_cast<size_t>(m.per) * 24;
+  const void* kr = invd ? reinterpret_cast<const void*>(&cg64_resident_kernel<true>)
+                        : reinterpret_cast<const void*>(&cg64_resident_kernel<false>);
+  const bool resident = m.per <= kResRows * kPT && smem <= kResSmem && resident_ok(A, kr);
+  void* params[] = {&a, &m};
   g_launches.fetch_add(1, std::memory_order_relaxed);
-  SK_CUDA(cudaLaunchCooperativeKernel(k, dim3(grid), dim3(kPT), params, 0, st));
+  SK_CUDA(cudaLaunchCooperativeKernel(resident ? kr : k, dim3(grid), dim3(kPT), params, resident ? smem : 0, st));
   int err = 0;
   SK_CUDA(cudaMemcpyAsync(&err, &sync->err, sizeof(int), cudaMemcpyDeviceToHost, st));
   SK_CUDA(cudaStreamSynchronize(st));
