@@ -184,6 +184,7 @@ struct Csr {
   int* sym_col = nullptr;
   float* sym_val = nullptr;
   int sym_dn = 0;
+  bool sym_dupper = false;  // A symmetric bit for bit, sym_dn 4 or 6: only the offsets > 0 are stored
   int sym_doff[kDiaMax] = {};
   float* sym_dval = nullptr;
   unsigned short* sym_dmask = nullptr;

@@ -398,7 +398,44 @@ __device__ __forceinline__ double phase_s_dia(PArgs const& a, int t0, int T, flo
   return pq;
 }
 
-template <bool DIA, bool UNIT>
+// Phase S with the number of diagonals known when it is compiled: every value
+// and every r of a row issued together (phase_s_dia waits once per kDiaGroup
+// diagonals).  SYM: S is symmetric and only its upper diagonals are stored;
+// A(i, i - o) is read where A(i - o, i) stands, so that the matrix is 12
+// instead of 24 bytes a row of a 7-point stencil, and with the five vectors
+// and the masks S stays in L2 at 2M rows: no evict-first hint.
+// 128^3 diffusion, whole mixed solve to 1e-10: 34.6 ms over groups of four
+// stored diagonals, 22.6 so.
+template <bool UNIT, bool FIRST, int ND, bool SYM>
+__device__ __forceinline__ double phase_s_planes(PArgs const& a, int t0, int T, float beta) {
+  constexpr int NL = SYM ? ND / 2 : 0, NP = ND - NL;
+  double pq = 0.0;
+  const int last = a.n - 1;
+  for (int i = t0; i < a.n; i += T) {
+    const unsigned m = __ldg(a.dia_mask + i);
+    const float ro = a.r[i], po = FIRST ? 0.0f : a.p[i], qo = FIRST ? 0.0f : a.q[i];
+    float v[ND], g[ND];
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
+      const int c = min(max(i + a.dia_off[d], 0), last);
+      const int row = d < NL ? c : i;
+      const int p = d < NL ? ND - 1 - d - NL : d - NL;
+      const float* at = a.val + (static_cast<long long>(row >> 5) * NP + p) * 32 + (row & 31);
+      v[d] = SYM ? __ldg(at) : __ldcs(at);
+      g[d] = a.r[c];
+    }
+    float s = UNIT ? ro : 0.0f;
+#pragma unroll
+    for (int d = 0; d < ND; ++d)
+      if ((m >> d) & 1u) s = add(s, mul(v[d], g[d]));
+    pq += row_direction<FIRST>(a, i, ro, s, po, qo, beta);
+  }
+  return pq;
+}
+
+// ND > 0: planes of ND diagonals (DIA), of which the upper half is stored when
+// SYM; ND = 0: any number, all stored.
+template <bool DIA, bool UNIT, int ND = 0, bool SYM = false>
 __global__ void __launch_bounds__(kPT, DIA ? 2 : 1) inner_cg_kernel(PArgs a) {
   const int n = a.n;
   const int T = gridDim.x * kPT;
@@ -435,10 +472,12 @@ __global__ void __launch_bounds__(kPT, DIA ? 2 : 1) inner_cg_kernel(PArgs a) {
   // phase S of one step (the first with p = r, q = A r) and <p, q>
   auto phase_s = [&](double (&pq)[1], bool first_step) -> bool {
     if (first_step) {
-      if constexpr (DIA) pq[0] = phase_s_dia<UNIT, true>(a, t0, T, beta);
+      if constexpr (ND > 0) pq[0] = phase_s_planes<UNIT, true, ND, SYM>(a, t0, T, beta);
+      else if constexpr (DIA) pq[0] = phase_s_dia<UNIT, true>(a, t0, T, beta);
       else pq[0] = phase_s_sell<UNIT, true>(a, t0, T, beta);
     } else {
-      if constexpr (DIA) pq[0] = phase_s_dia<UNIT, false>(a, t0, T, beta);
+      if constexpr (ND > 0) pq[0] = phase_s_planes<UNIT, false, ND, SYM>(a, t0, T, beta);
+      else if constexpr (DIA) pq[0] = phase_s_dia<UNIT, false>(a, t0, T, beta);
       else pq[0] = phase_s_sell<UNIT, false>(a, t0, T, beta);
     }
     return grid_allreduce<1, DIA>(pq, a, epoch);
@@ -510,7 +549,13 @@ __global__ void __launch_bounds__(kPT, DIA ? 2 : 1) inner_cg_kernel(PArgs a) {
   }
 }
 
-const void* pick_kernel(bool dia, bool unit) {
+const void* pick_kernel(sk_matrix A, bool dia, bool unit) {
+  if (dia && unit && A->csr.sym_dn == 6)  // 7-point stencils without their diagonal
+    return A->csr.sym_dupper ? reinterpret_cast<const void*>(&inner_cg_kernel<true, true, 6, true>)
+                             : reinterpret_cast<const void*>(&inner_cg_kernel<true, true, 6, false>);
+  if (dia && unit && A->csr.sym_dn == 4)  // 5-point
+    return A->csr.sym_dupper ? reinterpret_cast<const void*>(&inner_cg_kernel<true, true, 4, true>)
+                             : reinterpret_cast<const void*>(&inner_cg_kernel<true, true, 4, false>);
   if (dia)
     return unit ? reinterpret_cast<const void*>(&inner_cg_kernel<true, true>)
                 : reinterpret_cast<const void*>(&inner_cg_kernel<true, false>);
@@ -1389,7 +1434,8 @@ struct SymOffsets {
 
 __global__ void sym_dia_fill_kernel(i64 n, const int* __restrict__ rp, const int* __restrict__ ci,
                                     const double* __restrict__ v, const double* __restrict__ isq, SymOffsets o,
-                                    float* __restrict__ planes, unsigned short* __restrict__ mask) {
+                                    int first, float* __restrict__ planes, unsigned short* __restrict__ mask) {
+  const int np = o.n - first;  // the planes of the diagonals first .. o.n - 1 are stored
   for (i64 r = blockIdx.x * static_cast<i64>(blockDim.x) + threadIdx.x; r < n;
        r += static_cast<i64>(gridDim.x) * blockDim.x) {
     unsigned m = 0;
@@ -1400,7 +1446,7 @@ __global__ void sym_dia_fill_kernel(i64 n, const int* __restrict__ rp, const int
       const int off = c - static_cast<int>(r);
       int d = 0;
       while (d + 1 < o.n && o.off[d] != off) ++d;  // every off-diagonal offset is in the set
-      planes[((r >> 5) * o.n + d) * 32 + (r & 31)] = sym_value(v[k], sr, isq[c]);
+      if (d >= first) planes[((r >> 5) * np + d - first) * 32 + (r & 31)] = sym_value(v[k], sr, isq[c]);
       m |= 1u << d;
     }
     mask[r] = static_cast<unsigned short>(m);
@@ -1497,20 +1543,24 @@ sk_status sym_prepare_dia(sk_matrix A, cudaStream_t st) {
     C.sym_dia_state = -1;
     return SK_OK;
   }
-  const i64 len = (n + 31) / 32 * 32 * o.n;
-  void *planes = nullptr, *mask = nullptr;
   sk_status s;
+  bool upper = false;
+  if ((o.n == 4 || o.n == 6) && (s = csr_symmetric(A, offs, &upper)) != SK_OK) return s;
+  const int first = upper ? o.n / 2 : 0;
+  const i64 len = (n + 31) / 32 * 32 * (o.n - first);
+  void *planes = nullptr, *mask = nullptr;
   if ((s = dev_alloc(A, &planes, len * 4 + 64)) != SK_OK) return s;
   if ((s = dev_alloc(A, &mask, (n + 64) * 2)) != SK_OK) return s;
   SK_CUDA(cudaMemsetAsync(planes, 0, len * 4 + 64, st));
   SK_LAUNCH(sym_dia_fill_kernel, grid_for(n), kThreads, 0, st, n, C.row_ptr, C.col_ind,
-            static_cast<const double*>(C.vals), C.sym_isq, o, static_cast<float*>(planes),
+            static_cast<const double*>(C.vals), C.sym_isq, o, first, static_cast<float*>(planes),
             static_cast<unsigned short*>(mask));
   SK_CUDA(cudaGetLastError());
   SK_CUDA(cudaStreamSynchronize(st));
   C.sym_dval = static_cast<float*>(planes);
   C.sym_dmask = static_cast<unsigned short*>(mask);
   C.sym_dn = o.n;
+  C.sym_dupper = upper;
   for (int k = 0; k < o.n; ++k) C.sym_doff[k] = o.off[k];
   C.sym_dia_state = 1;
   return SK_OK;
@@ -1548,7 +1598,7 @@ bool inner_persistent_ok(sk_matrix A, bool scaled) {
   if (A->nrow > INT_MAX / 4) return false;
   int coop = 0;
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, A->device) != cudaSuccess || !coop) return false;
-  return coop_grid(A, pick_kernel(use_dia(A, scaled), scaled)) > 0;
+  return coop_grid(A, pick_kernel(A, use_dia(A, scaled), scaled)) > 0;
 }
 
 size_t inner_persistent_scratch(sk_matrix) {
@@ -1565,7 +1615,7 @@ sk_status inner_cg_persistent(sk_matrix A, bool scaled, float* r, float* d, floa
            scaled ? "persistent scaled inner solve: the scaled copy is not built"
                   : "persistent inner solve needs a CSR handle with FP32 SELL values or an FP32 diagonal copy");
   const bool dia = use_dia(A, scaled);
-  const void* k = pick_kernel(dia, scaled);
+  const void* k = pick_kernel(A, dia, scaled);
   int grid = coop_grid(A, k);
   SK_CHECK(grid > 0, SK_NOT_SUPPORTED, "persistent inner solve does not fit on the device");
   grid = std::min(grid, kPT);  // the slots' size
