@@ -102,6 +102,25 @@ def _stream_of(a):
     return None
 
 
+def _plain_vectors(a, na, b, nb, dtype, device):
+    """(pointer of a, pointer of b, stream) when both are what _check_vec asks
+    for, plain tensors on `device`; None sends the call through the checks one
+    by one, which say what is wrong.  A small product takes 3 us on the device
+    and the checks took 6 on the host; these take 1.5."""
+    import torch
+    T = torch.Tensor
+    if a.__class__ is not T or b.__class__ is not T or device is None:
+        return None
+    want = torch.float64 if dtype.itemsize == 8 else torch.float32
+    if (a.dtype is not want or b.dtype is not want or a.numel() != na or b.numel() != nb or not a.is_contiguous()
+            or not b.is_contiguous() or not a.is_cuda or not b.is_cuda or a.get_device() != device
+            or b.get_device() != device):
+        return None
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # without a Stream object, 1 us less
+    st = raw(device) if raw is not None else torch.cuda.current_stream(device).cuda_stream
+    return a.data_ptr(), b.data_ptr(), st or CUDA_STREAM_LEGACY
+
+
 class Device_matrix:
     """A device-resident copy of one reference matrix object."""
 
@@ -219,6 +238,10 @@ class Device_matrix:
         """y = A x on device tensors (or raw device pointers, which the
         caller vouches for)."""
         n, m = self._shape
+        plain = _plain_vectors(x, m, y, n, self.dtype, self.device) if stream is None else None
+        if plain is not None:
+            check(lib().sk_spmv(self.handle, *plain))
+            return
         if not isinstance(x, int):
             _check_vec(x, m, self.dtype, self.device, "x")
         if not isinstance(y, int):
@@ -319,6 +342,10 @@ class _Precond:
 
     def apply(self, r, z, stream=None):
         """z = M^{-1} r on device tensors."""
+        plain = _plain_vectors(r, self.n, z, self.n, self.A.dtype, self.A.device) if stream is None else None
+        if plain is not None:
+            check(lib().sk_precond_apply(self.handle, self.n, *plain))
+            return
         _check_vec(r, self.n, self.A.dtype, self.A.device, "r")
         _check_vec(z, self.n, self.A.dtype, self.A.device, "z")
         st = stream if stream is not None else _stream_of(r)
