@@ -394,15 +394,22 @@ struct ConvSmem {
 // upsample-and-add loads and stores.  FEAT: the first layer of an apply
 // (8 input channels, one sample) computes channel 0 of its input, the
 // scaled vector v / d / s, into the staged planes itself; the other
-// channels come from a tensor that holds the matrix's fixed features.
-template <int CIN, int N, bool TC, bool UP, int TM = 1, int CS = 1, bool FEAT = false>
+// channels come from a tensor that holds the matrix's fixed features.  NS:
+// CTAs per tile (tcgen05 only), each with N / NS of its output channels and
+// their weights, for layers with fewer tiles than SMs: what bounds those is
+// the chain of one CTA, of which the epilogue, NS times shorter, is half.
+// Apply at 512^2 (split: the two 64^2 layers): 96.4 us before, 88.4 so; at
+// 56 x 288 (all but the full-resolution layers): 62.7 and 49.0.
+template <int CIN, int N, bool TC, bool UP, int TM = 1, int CS = 1, bool FEAT = false, int NS = 1>
 __global__ void __launch_bounds__(kConvThreads * CS) conv3x3_kernel(const __grid_constant__ CUtensorMap in_map,
                                                                     ConvArgs a) {
   static_assert(TC || TM == 1, "several tiles per CTA only on the tcgen05 path");
   static_assert(!FEAT || (CIN == 8 && TC), "fused features only for the first layer on the tcgen05 path");
   static_assert(CS == 1 || (TC && N / CS >= 16), "channel split only on the tcgen05 path, 16 columns or more");
-  constexpr int NC = N / CS;
-  using S = ConvSmem<CIN, N, TC, TM>;
+  static_assert(NS == 1 || (TC && CS == 1 && N / NS >= 16), "split tiles only on the tcgen05 path");
+  constexpr int NW = N / NS;  // output channels of this CTA
+  constexpr int NC = NW / CS;
+  using S = ConvSmem<CIN, NW, TC, TM>;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* planes = smem + S::kIn;
   unsigned char* wsm = smem + S::kW;
@@ -413,9 +420,11 @@ __global__ void __launch_bounds__(kConvThreads * CS) conv3x3_kernel(const __grid
   __shared__ float s_bias[N];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int px = tid & (kConvThreads - 1), cbase = (tid / kConvThreads) * NC;  // pixel, first channel
-  const int x0 = blockIdx.x * kTileW * TM, y0 = blockIdx.y * kTileH, b = blockIdx.z;
-  constexpr uint32_t kCols = TM * N < 32 ? 32 : TM * N;
+  const int n0 = NS == 1 ? 0 : static_cast<int>(blockIdx.z % NS) * NW;
+  const int px = tid & (kConvThreads - 1), cacc = (tid / kConvThreads) * NC;  // pixel, first accumulator
+  const int cbase = n0 + cacc;                                                // first channel
+  const int x0 = blockIdx.x * kTileW * TM, y0 = blockIdx.y * kTileH, b = blockIdx.z / NS;
+  constexpr uint32_t kCols = TM * NW < 32 ? 32 : TM * NW;
 
   // Launched as a programmatic dependent of the previous layer: this CTA
   // sets up (barriers, tensor memory), then lets the next layer launch, and
@@ -442,9 +451,14 @@ __global__ void __launch_bounds__(kConvThreads * CS) conv3x3_kernel(const __grid
   // the previous layer's output: they wait for it.
   // (a single-channel output has one bias value)
   if (tid < N) s_bias[tid] = a.bias && (a.out_kind == OUT_BF16 || tid == 0) ? __ldg(a.bias + tid) : 0.0f;
-  if (tid == 0) {
-    mbar_expect_tx(bar_load, TM * S::kPlanes * kPlaneBytes + S::kWBytes);
-    bulk_load(wsm, a.wpk, S::kWBytes, bar_load);
+  if (tid == 0) mbar_expect_tx(bar_load, TM * S::kPlanes * kPlaneBytes + S::kWBytes);
+  if constexpr (NS == 1) {
+    if (tid == 0) bulk_load(wsm, a.wpk, S::kWBytes, bar_load);
+  } else {  // this CTA's channels of every 8-channel input chunk: 16 bytes each, side by side
+    __syncwarp();
+    if (warp == 0)
+      for (int k = lane; k < S::kKC; k += 32)
+        bulk_load(wsm + k * NW * 16, a.wpk + (static_cast<size_t>(k) * N + n0) * 8, NW * 16, bar_load);
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (tid == 0) {
@@ -513,7 +527,7 @@ __global__ void __launch_bounds__(kConvThreads * CS) conv3x3_kernel(const __grid
     if (tid == 0 && ok) {
 #pragma unroll
       for (int t = 0; t < TM; ++t)
-        conv_issue_mma<CIN, N>(smem_u32(planes) + t * S::kPlanes * kPlaneStride, smem_u32(wsm), tmem + t * N);
+        conv_issue_mma<CIN, NW>(smem_u32(planes) + t * S::kPlanes * kPlaneStride, smem_u32(wsm), tmem + t * NW);
       umma_commit(bar_mma);
     }
     __syncthreads();
@@ -527,7 +541,7 @@ __global__ void __launch_bounds__(kConvThreads * CS) conv3x3_kernel(const __grid
 #pragma unroll
       for (int c = 0; c < NC / 16; ++c) {
         float u[16];
-        tmem_ld16(row + t * N + cbase + c * 16, u);
+        tmem_ld16(row + t * NW + cacc + c * 16, u);
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < 16; ++j) v[c * 16 + j] = u[j];
@@ -1168,6 +1182,7 @@ struct MapCache {
 // More tiles than this many CTAs per SM could hold at once: the layers
 // with 16 output channels take two tiles per CTA (one wave instead of two).
 constexpr int kConvWaveCtas = 8 * 148;
+constexpr int kConvSplitCtas = 148;  // most CTAs of a layer whose tiles are split by output channels
 
 template <int CIN, int N, bool TC>
 static sk_status launch_conv(MapCache& mc, const void* in, ConvArgs const& a, cudaStream_t st) {
@@ -1185,8 +1200,21 @@ static sk_status launch_conv(MapCache& mc, const void* in, ConvArgs const& a, cu
       bytes = ConvSmem<CIN, N, TC, 2>::kBytes;
     }
   }
-  if constexpr (TC && N >= 32) {  // the upsample-and-add epilogue split over two threads per pixel
-    if (a.up_out) {
+  int ns = 1;
+  if constexpr (TC && N >= 32) {
+    // while every CTA has an SM to itself, the channels over CTAs, 16 each;
+    // else the upsample-and-add epilogue over two threads per pixel
+    if (ntiles * (N / 16) <= kConvSplitCtas) {
+      ns = N / 16;
+      kernel = a.up_out ? conv3x3_kernel<CIN, N, TC, true, 1, 1, false, N / 16>
+                        : conv3x3_kernel<CIN, N, TC, false, 1, 1, false, N / 16>;
+      bytes = ConvSmem<CIN, 16, TC>::kBytes;
+    } else if (N == 64 && ntiles * 2 <= kConvSplitCtas) {
+      ns = 2;
+      kernel = a.up_out ? conv3x3_kernel<CIN, N, TC, true, 1, 1, false, 2>
+                        : conv3x3_kernel<CIN, N, TC, false, 1, 1, false, 2>;
+      bytes = ConvSmem<CIN, N / 2, TC>::kBytes;
+    } else if (a.up_out) {
       cs = 2;
       kernel = conv3x3_kernel<CIN, N, TC, true, 1, 2>;
     }
@@ -1207,7 +1235,7 @@ static sk_status launch_conv(MapCache& mc, const void* in, ConvArgs const& a, cu
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   const int ntx = ceil_div(a.W, kTileW * tm), nty = ceil_div(a.H, kTileH);
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(ntx, nty, a.B);
+  cfg.gridDim = dim3(ntx, nty, a.B * ns);
   cfg.blockDim = dim3(kConvThreads * cs);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
@@ -1653,6 +1681,16 @@ static sk_status conv_attrs() {
     SK_CONV_ATTR_CS(64, 32)
     SK_CONV_ATTR_CS(64, 64)
 #undef SK_CONV_ATTR_CS
+#define SK_CONV_ATTR_NS(CI, NN, K)                                                                        \
+  ok = ok && attr_once(conv3x3_kernel<CI, NN, TC, false, 1, 1, false, K>, ConvSmem<CI, NN / K, TC>::kBytes) && \
+       attr_once(conv3x3_kernel<CI, NN, TC, true, 1, 1, false, K>, ConvSmem<CI, NN / K, TC>::kBytes);
+    SK_CONV_ATTR_NS(16, 32, 2)
+    SK_CONV_ATTR_NS(32, 64, 4)
+    SK_CONV_ATTR_NS(32, 64, 2)
+    SK_CONV_ATTR_NS(64, 32, 2)
+    SK_CONV_ATTR_NS(64, 64, 4)
+    SK_CONV_ATTR_NS(64, 64, 2)
+#undef SK_CONV_ATTR_NS
   }
   SK_CONV_ATTR(8, 16)
   SK_CONV_ATTR(16, 16)
