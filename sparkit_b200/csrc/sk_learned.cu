@@ -731,21 +731,40 @@ __global__ void __launch_bounds__(kConvThreads) wgrad_kernel(const __grid_consta
 }
 
 // grad[w_off + (co * 9 + t) * CI + ci] = sum_k part[t][k][co][ci] (k in
-// order); grad[b_off + co] = sum_k bpart[k][co]; co < cout_true only.
-__global__ void wgrad_reduce_kernel(const float* part, const float* bpart, int nctas, int CO, int CI, int cout_true,
-                                    float* grad_w, float* grad_b) {
-  const int total = 9 * cout_true * CI;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total + cout_true; i += gridDim.x * blockDim.x) {
+// order); grad[b_off + co] = sum_k bpart[k][co]; co < cout_true only.  Layer l
+// is blockIdx.y; a thread's partials are loaded eight at a time.
+struct WgradReduceLayer {
+  const float* part;
+  const float* bpart;
+  int nctas, CO, CI, cout_true;
+  float* grad_w;
+  float* grad_b;
+};
+struct WgradReduceArgs {
+  WgradReduceLayer l[kNL];
+};
+__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const __grid_constant__ WgradReduceArgs a) {
+  const WgradReduceLayer& L = a.l[blockIdx.y];
+  const int total = 9 * L.cout_true * L.CI;
+  auto sum = [&](const float* p, size_t stride) {
+    float s = 0.0f;
+    for (int k0 = 0; k0 < L.nctas; k0 += 8) {
+      float v[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) v[k] = k0 + k < L.nctas ? p[(k0 + k) * stride] : 0.0f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        if (k0 + k < L.nctas) s += v[k];
+    }
+    return s;
+  };
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total + L.cout_true; i += gridDim.x * blockDim.x) {
     if (i < total) {
-      const int ci = i % CI, t = (i / CI) % 9, co = i / (CI * 9);
-      float s = 0.0f;
-      for (int k = 0; k < nctas; ++k) s += part[((static_cast<size_t>(t) * nctas + k) * CO + co) * CI + ci];
-      grad_w[i] = s;
+      const int ci = i % L.CI, t = (i / L.CI) % 9, co = i / (L.CI * 9);
+      const size_t step = static_cast<size_t>(L.CO) * L.CI;
+      L.grad_w[i] = sum(L.part + t * L.nctas * step + static_cast<size_t>(co) * L.CI + ci, step);
     } else {
-      const int co = i - total;
-      float s = 0.0f;
-      for (int k = 0; k < nctas; ++k) s += bpart[static_cast<size_t>(k) * CO + co];
-      grad_b[co] = s;
+      L.grad_b[i - total] = sum(L.bpart + (i - total), L.CO);
     }
   }
 }
@@ -949,17 +968,21 @@ __global__ void __launch_bounds__(kThreads) loss1_kernel(LossArgs a) {
     last = atomicAdd(a.counter + b, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (last && threadIdx.x == 0) {
+  if (last) {  // the last CTA sums the partials with all its threads (a fixed tree; one thread took 30 us)
     __threadfence();
     double t[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int k = 0; k < static_cast<int>(gridDim.x); ++k)
+    for (int k = threadIdx.x; k < static_cast<int>(gridDim.x); k += blockDim.x)
+#pragma unroll
       for (int j = 0; j < 4; ++j) t[j] += __ldcg(a.partial + (b * kRedBlocks + k) * 4 + j);
-    const double wr = t[1] > 0.0 ? 1.0 / t[1] : 0.0;
-    const double wt = t[2] > 0.0 ? a.mu / t[2] : 0.0;
-    a.wts[b * 3 + 0] = wr;
-    a.wts[b * 3 + 1] = wt;
-    a.wts[b * 3 + 2] = t[0] * wr + t[3] * wt;
-    a.counter[b] = 0u;
+    block_reduce<4>(t);
+    if (threadIdx.x == 0) {
+      const double wr = t[1] > 0.0 ? 1.0 / t[1] : 0.0;
+      const double wt = t[2] > 0.0 ? a.mu / t[2] : 0.0;
+      a.wts[b * 3 + 0] = wr;
+      a.wts[b * 3 + 1] = wt;
+      a.wts[b * 3 + 2] = t[0] * wr + t[3] * wt;
+      a.counter[b] = 0u;
+    }
   }
 }
 
@@ -1329,7 +1352,14 @@ struct sk_net_s {
   double *s, *red, *wts, *loss;
   unsigned* counter;
   float *part, *bpart;
-  int wg_ctas = 0;
+  // Weight gradients run on `side`, beside the chain of input gradients: layer
+  // l's partials start at part_off[l] / bpart_off[l], of wg_ctas[l] CTAs.
+  size_t part_off[kNL] = {}, bpart_off[kNL] = {};
+  int wg_ctas[kNL] = {};
+  cudaStream_t side = nullptr;
+  cudaEvent_t ready = nullptr, done = nullptr;
+  int* idx = nullptr;  // pair indices of sk_net_loss_grad
+  int idx_cap = 0;
   std::vector<void*> allocs;
 };
 
@@ -1353,13 +1383,27 @@ static sk_status net_alloc(sk_net N, void** p, size_t bytes) {
   return SK_OK;
 }
 
+constexpr int kWgCtas = 64;
+
 // Carves the workspace of a (B, H, W) configuration (grow-only).
 static sk_status net_workspace(sk_net N, int B, int H, int W) {
   if (N->B == B && N->H == H && N->W == W && N->ws) return SK_OK;
   SK_CHECK(H % 8 == 0 && W % 8 == 0 && H >= 8 && W >= 8, SK_INVALID_ARG, "grid sides must be multiples of 8");
   const size_t P0 = static_cast<size_t>(B) * H * W, P1 = P0 / 4, P2 = P0 / 16, P3 = P0 / 64;
   struct Item { void** dst; size_t bytes; };
-  const int ctas = 2 * 148;
+  // A layer's tiles are split over at most kWgCtas CTAs per tap (9 taps: four
+  // CTAs to an SM, whose tile copies hide behind one another)
+  static const int level[kNL] = {0, 1, 2, 3, 3, 2, 1, 0, 0};
+  size_t parts = 0, bparts = 0, part_off[kNL], bpart_off[kNL];
+  int ctas[kNL];
+  for (int l = 0; l < kNL; ++l) {
+    const int tiles = ceil_div(W >> level[l], kTileW) * ceil_div(H >> level[l], kTileH) * B;
+    ctas[l] = std::min(kWgCtas, tiles);
+    part_off[l] = parts;
+    bpart_off[l] = bparts;
+    parts += static_cast<size_t>(9) * ctas[l] * pad_n(kCout[l]) * kCin[l];
+    bparts += static_cast<size_t>(ctas[l]) * pad_n(kCout[l]);
+  }
   std::vector<Item> items = {
       {(void**)&N->x0, P0 * 8 * 2},   {(void**)&N->e0, P0 * 16 * 2}, {(void**)&N->p0, P1 * 16 * 2},
       {(void**)&N->e1, P1 * 32 * 2},  {(void**)&N->p1, P2 * 32 * 2}, {(void**)&N->e2, P2 * 64 * 2},
@@ -1375,8 +1419,8 @@ static sk_status net_workspace(sk_net N, int B, int H, int W) {
       {(void**)&N->red, static_cast<size_t>(B) * kRedBlocks * 4 * 8},
       {(void**)&N->wts, static_cast<size_t>(B) * 3 * 8},              {(void**)&N->loss, 8},
       {(void**)&N->counter, static_cast<size_t>(B) * 4},
-      {(void**)&N->part, static_cast<size_t>(9) * ctas * 64 * 64 * 4},
-      {(void**)&N->bpart, static_cast<size_t>(ctas) * 64 * 4}};
+      {(void**)&N->part, parts * 4},
+      {(void**)&N->bpart, bparts * 4}};
   size_t total = 0;
   for (auto& it : items) total += (it.bytes + 255) & ~size_t(255);
   if (total > N->ws_bytes) {
@@ -1398,7 +1442,9 @@ static sk_status net_workspace(sk_net N, int B, int H, int W) {
   N->B = B;
   N->H = H;
   N->W = W;
-  N->wg_ctas = ctas;
+  std::copy(ctas, ctas + kNL, N->wg_ctas);
+  std::copy(part_off, part_off + kNL, N->part_off);
+  std::copy(bpart_off, bpart_off + kNL, N->bpart_off);
   return SK_OK;
 }
 
@@ -1456,25 +1502,36 @@ static sk_status run_dgrad(sk_net N, int l, const bf16* g, int H, int W, bf16* o
                        : conv_dispatch<true>(N->maps, cin, kCin[l], g, a, N->stream);
 }
 
+// The weight gradient of layer l, on the side stream once what N->stream holds
+// now (x and g) is done.
 static sk_status run_wgrad(sk_net N, int l, const bf16* x, const bf16* g, int H, int W) {
+  SK_CUDA(cudaEventRecord(N->ready, N->stream));
+  SK_CUDA(cudaStreamWaitEvent(N->side, N->ready, 0));
   WgradArgs a{};
   a.B = N->B;
   a.H = H;
   a.W = W;
   a.ntiles_x = ceil_div(W, kTileW);
   a.ntiles_y = ceil_div(H, kTileH);
-  a.part = N->part;
-  a.bpart = N->bpart;
+  a.part = N->part + N->part_off[l];
+  a.bpart = N->bpart + N->bpart_off[l];
   a.err = N->err;
-  const int ntiles = a.ntiles_x * a.ntiles_y * a.B;
-  const int nctas = std::min(N->wg_ctas / 9 + 1, ntiles);
-  const int co = pad_n(kCout[l]);
-  sk_status s = wgrad_dispatch(N->maps, kCin[l], co, x, g, a, nctas, N->stream);
-  if (s != SK_OK) return s;
-  const int total = 9 * kCout[l] * kCin[l] + kCout[l];
-  SK_LAUNCH(wgrad_reduce_kernel, ceil_div(total, 256), 256, 0, N->stream, N->part, N->bpart, nctas, co, kCin[l],
-            kCout[l], N->grad + N->w_off[l], N->grad + N->b_off[l]);
+  return wgrad_dispatch(N->maps, kCin[l], pad_n(kCout[l]), x, g, a, N->wg_ctas[l], N->side);
+}
+
+// The sum of every layer's partials, after which N->stream goes on.
+static sk_status finish_wgrad(sk_net N) {
+  WgradReduceArgs a{};
+  int most = 0;
+  for (int l = 0; l < kNL; ++l) {
+    a.l[l] = {N->part + N->part_off[l], N->bpart + N->bpart_off[l], N->wg_ctas[l], pad_n(kCout[l]), kCin[l], kCout[l],
+              N->grad + N->w_off[l], N->grad + N->b_off[l]};
+    most = std::max(most, 9 * kCout[l] * kCin[l] + kCout[l]);
+  }
+  SK_LAUNCH(wgrad_reduce_kernel, dim3(ceil_div(most, 256), kNL), 256, 0, N->side, a);
   SK_CUDA(cudaGetLastError());
+  SK_CUDA(cudaEventRecord(N->done, N->side));
+  SK_CUDA(cudaStreamWaitEvent(N->stream, N->done, 0));
   return SK_OK;
 }
 
@@ -1545,8 +1602,7 @@ static sk_status net_backward(sk_net N) {
   SK_LAUNCH(pool_bwd_kernel, ew_grid(static_cast<i64>(B) * H * W * 2), 256, 0, st, B, H, W, 16, N->du0, N->dp0,
             N->e0, N->g0);
   if ((s = run_wgrad(N, 0, N->x0, N->g0, H, W)) != SK_OK) return s;
-  SK_CUDA(cudaGetLastError());
-  return SK_OK;
+  return finish_wgrad(N);
 }
 
 static sk_status check_err(sk_net N) {
@@ -1560,9 +1616,15 @@ static sk_status check_err(sk_net N) {
   return SK_OK;
 }
 
+// CTAs of a reduction over P cells: one cell a thread, kRedBlocks at most
+// (the partials of CTAs without a cell were zeros: the same sums).
+static unsigned red_blocks(i64 P) {
+  return static_cast<unsigned>(std::max<i64>(1, std::min<i64>(kRedBlocks, (P + kThreads - 1) / kThreads)));
+}
+
 // features of a batch into N->x0 (and scales into N->s)
 static void net_features(sk_net N, SampleSrc const& src, int B) {
-  SK_LAUNCH(scale_kernel, dim3(kRedBlocks, B), kThreads, 0, N->stream, src, N->red, N->counter, N->s);
+  SK_LAUNCH(scale_kernel, dim3(red_blocks(src.P), B), kThreads, 0, N->stream, src, N->red, N->counter, N->s);
   SK_LAUNCH(features_kernel, ew_grid(static_cast<i64>(B) * src.P), 256, 0, N->stream, src, B, N->s, N->x0);
 }
 
@@ -1582,7 +1644,7 @@ static void net_loss(sk_net N, SampleSrc const& src, double mu, double* loss_out
   a.mu = mu;
   a.g8 = N->g8;
   a.loss_out = loss_out;
-  SK_LAUNCH(loss1_kernel, dim3(kRedBlocks, N->B), kThreads, 0, N->stream, a);
+  SK_LAUNCH(loss1_kernel, dim3(red_blocks(src.P), N->B), kThreads, 0, N->stream, a);
   SK_LAUNCH(loss2_kernel, ew_grid(static_cast<i64>(N->B) * src.P), 256, 0, N->stream, a);
 }
 
@@ -1642,7 +1704,7 @@ sk_status learned_apply_ex(const sk_precond_s* M, const double* v, double* z, cu
   src.coef = M->coef;
   src.P = M->n;
   if (!scale_ready)
-    SK_LAUNCH(scale_kernel, dim3(kRedBlocks, 1), kThreads, 0, N->stream, src, N->red, N->counter, N->s);
+    SK_LAUNCH(scale_kernel, dim3(red_blocks(src.P), 1), kThreads, 0, N->stream, src, N->red, N->counter, N->s);
   ConvArgs last{};
   last.out_kind = OUT_Z64;
   last.outz = z;
@@ -1757,6 +1819,10 @@ sk_status sk_net_create(sk_net* out, uint64_t seed) {
     }
   }
   if ((s = net_alloc(N, reinterpret_cast<void**>(&N->err), 16)) != SK_OK) return bail(s);
+  if (cudaStreamCreateWithFlags(&N->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&N->ready, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&N->done, cudaEventDisableTiming) != cudaSuccess)
+    return bail(fail(SK_CUDA_ERROR, "network streams"));
   // He initialisation (normal, std sqrt(2 / fan_in)), zero biases
   std::vector<float> h(N->np, 0.0f);
   std::mt19937_64 rng(seed);
@@ -1780,6 +1846,10 @@ sk_status sk_net_destroy(sk_net N) {
   cudaDeviceSynchronize();
   for (void* p : N->allocs) cudaFree(p);
   if (N->ws) cudaFree(N->ws);
+  if (N->idx) cudaFree(N->idx);
+  if (N->ready) cudaEventDestroy(N->ready);
+  if (N->done) cudaEventDestroy(N->done);
+  if (N->side) cudaStreamDestroy(N->side);
   delete N;
   return SK_OK;
 }
@@ -1942,8 +2012,14 @@ sk_status sk_net_loss_grad(sk_net N, sk_pairs D, const int32_t* pairs_host, int3
   SK_CHECK(N && D && pairs_host && loss && batch >= 1, SK_INVALID_ARG, "null argument");
   for (int b = 0; b < batch; ++b)
     SK_CHECK(pairs_host[b] >= 0 && pairs_host[b] < D->count, SK_INVALID_ARG, "pair index out of range");
-  int* idx = nullptr;
-  SK_CUDA(cudaMalloc(&idx, batch * 4));
+  if (batch > N->idx_cap) {
+    if (N->idx) cudaFree(N->idx);
+    N->idx = nullptr;
+    N->idx_cap = 0;
+    SK_CUDA(cudaMalloc(&N->idx, batch * 4));
+    N->idx_cap = batch;
+  }
+  int* idx = N->idx;
   SK_CUDA(cudaMemcpy(idx, pairs_host, batch * 4, cudaMemcpyHostToDevice));
   N->stream = nullptr;
   sk_status s = net_workspace(N, batch, D->ny, D->nx);  // N->loss lives in it
@@ -1953,7 +2029,6 @@ sk_status sk_net_loss_grad(sk_net N, sk_pairs D, const int32_t* pairs_host, int3
     cudaMemcpy(loss, N->loss, 8, cudaMemcpyDeviceToHost);
     if (grad_host && capacity >= N->np) cudaMemcpy(grad_host, N->grad, N->np * 4, cudaMemcpyDeviceToHost);
   }
-  cudaFree(idx);
   return s;
 }
 
