@@ -880,15 +880,6 @@ static sk_status bicgstab_solve(sk_matrix A, sk_precond L, sk_precond R, const T
 // FGMRES(m), fgmres.hpp:96-428
 // ==================================================================
 
-struct FgSmall {  // device arrays of one restart cycle
-  double* H;   // (m+1) x m, column-major, leading dimension m+1
-  double* cs;
-  double* sn;
-  double* g;   // m+1
-  double* y;   // m
-  double* zero;  // a constant 0 (the h of an MGS pass that only takes a dot)
-};
-
 // GMRES(m) (gmres.hpp:106-396) runs the FGMRES cycle with these changes:
 // the left preconditioner M_L on the initial residual and on A z_j
 // (:221-222, :253-254), and normalisation by division (:230, :278) where
@@ -1014,6 +1005,16 @@ struct EpiFgW {
     red[0] += static_cast<double>(mul(v0[row], val));
   }
   __device__ void finalize(const double* t) const { *h_out = static_cast<double>(static_cast<T>(t[0])); }
+};
+
+// The same product for the two-sum Gram-Schmidt, which takes every dot itself.
+template <typename T>
+struct EpiFgWStore {
+  static constexpr int kNR = 0;
+  T* w;
+  const T* linv;
+  __device__ void operator()(int row, T val, double*) const { w[row] = linv ? mul(linv[row], val) : val; }
+  __device__ void finalize(const double*) const {}
 };
 
 // orthogonalize (:259-273) step i: w -= h_ij v_i, then the next dot
@@ -1239,7 +1240,8 @@ static sk_status fgmres_solve(sk_matrix A, sk_precond M, const T* b, T* x,
   char* extra = nullptr;
   const i64 hist_cap = cfg->collect_residuals ? cfg->max_iterations : 0;
   // the Arnoldi step's barrier words and reduction slots (2 x grid <= 2 x 512)
-  const size_t arn_bytes = 256 + 2 * 512 * sizeof(double);
+  // and the two-sum form's workspace
+  const size_t arn_bytes = 256 + 2 * 512 * sizeof(double) + kArnLowBytes + 256;
   sk_status s = carve_common(A, st, 0, 0,
                              static_cast<size_t>(nvecs) * ldv * sizeof(T) + small_bytes + arn_bytes + 1024,
                              hist_cap, &c, &vv, &extra);
@@ -1264,7 +1266,11 @@ static sk_status fgmres_solve(sk_matrix A, sk_precond M, const T* b, T* x,
       (reinterpret_cast<uintptr_t>(smallp) + small_bytes + 255) & ~uintptr_t(255));
   double* arn_slots = reinterpret_cast<double*>(reinterpret_cast<char*>(arn_sync) + 256);
   sk_status arn_status = SK_OK;
-  if (arnoldi_fused) SK_CUDA(cudaMemsetAsync(arn_sync, 0, sizeof(ArnoldiSync), st));
+  auto* arn_box1 = reinterpret_cast<ulonglong2*>(arn_slots + 2 * 512);
+  auto* arn_box2 = arn_box1 + 2 * kArnLowCols * kArnLowGrid;
+  auto* arn_tri = reinterpret_cast<double*>(arn_box2 + 2 * kArnLowCols * kArnLowGrid);
+  if (arnoldi_fused)  // no tag of an earlier solve is left in a mailbox
+    SK_CUDA(cudaMemsetAsync(arn_sync, 0, aplan.low_grid ? arn_bytes - 256 : sizeof(ArnoldiSync), st));
   *out = sk_summary{};
   double bnorm = 0;
   if ((s = norm_b<T>(b, n, c, st, &bnorm)) != SK_OK) return s;
@@ -1302,14 +1308,19 @@ static sk_status fgmres_solve(sk_matrix A, sk_precond M, const T* b, T* x,
       if (general_left) {  // v_{j+1} = M_L A z_j, then h_0j = <v_0, v_{j+1}>
         launch_spmv<T>(A, Zj, EpiStore<T>{gl.tmp}, c.ws, c.sc, q, vals);
         precond_apply_dispatch(gl.L, kVecType<T>, n, gl.tmp, Vj1, c.ws, c.sc, q);
-        launch_vec(n, OpFgMgs<T>{Vj1, V, V, sm.zero, sm.H + j * um1, T(0)}, c.ws, c.sc, q);
+        if (!(arnoldi_fused && aplan.low(j)))
+          launch_vec(n, OpFgMgs<T>{Vj1, V, V, sm.zero, sm.H + j * um1, T(0)}, c.ws, c.sc, q);
+      } else if (arnoldi_fused && aplan.low(j)) {
+        launch_spmv<T>(A, Zj, EpiFgWStore<T>{Vj1, gl.linv}, c.ws, c.sc, q, vals);
       } else {
         launch_spmv<T>(A, Zj, EpiFgW<T>{Vj1, V, sm.H + j * um1, gl.linv}, c.ws, c.sc, q, vals);
       }
       if (arnoldi_fused) {
         const sk_status as = arnoldi_launch<T>(
-            aplan, ArnoldiArgs<T>{n, Vj1, V, ldv, j, sm.H + j * um1, gl.divide, c.sc, arn_sync, arn_slots, 0}, q);
+            aplan, ArnoldiArgs<T>{n, Vj1, V, ldv, j, sm.H + j * um1, gl.divide, c.sc, arn_sync, arn_slots, arn_box1,
+                                  arn_box2, arn_tri, c.sc, c.hist, sm, m, hess64, 0}, q);
         if (as != SK_OK && arn_status == SK_OK) arn_status = as;
+        if (aplan.low(j)) continue;  // with the rotations
       } else {
         for (int i = 0; i <= j; ++i) {
           const T* vnext = i < j ? V + (i + 1) * ldv : nullptr;

@@ -226,6 +226,34 @@ def test_gmres_matches_oracle_history(gpu_lib, oracle):
     assert np.linalg.norm(x - xr) <= 1e-8 * np.linalg.norm(xr)
 
 
+@pytest.mark.parametrize("n", [5, 63, 65, 1000, 148 * 64 + 1, 20011])
+@pytest.mark.parametrize("m", [6, 33, 70])
+def test_arnoldi_two_sum_form(gpu_lib, oracle, n, m):
+    """The Gram-Schmidt step behind two grid-wide sums: one CTA, a CTA that
+    holds one row, ragged rows, fewer and more basis vectors than warps, and a
+    cycle that goes on past the columns it takes.  The per-step estimates
+    |g_{j+1}| follow the oracle's modified Gram-Schmidt to the rounding of the
+    dot products, which is relative to ||b||."""
+    A = matgen.tridiagonal_matrix(n, -1.05, 2.1, -1.0)
+    b = oracle.spmv(A, matgen.uniform_vector(n, seed=5))
+    Ad = gpu.Device_matrix(A)
+    its = min(m + 7, n)
+    for solver in ("gmres", "fgmres"):
+        x = np.zeros(n)
+        if solver == "gmres":
+            J = gpu.jacobi(Ad)
+            s = gpu.gmres(b, x, gpu.Gmres_config(1e-15, m, its, True), gpu.spmv(Ad), left=J)
+            xr, sr = oracle.gmres(A, b, np.zeros(n), 1e-15, m, its, left="jacobi", collect=True)
+        else:
+            s = gpu.fgmres(b, x, gpu.Fgmres_config(1e-15, m, its, True), gpu.spmv(Ad))
+            xr, sr = oracle.fgmres(A, b, np.zeros(n), 1e-15, m, its, collect=True)
+        h, hr = np.array(s.iteration_residuals), np.array(sr["iteration_residuals"])
+        k = min(h.size, hr.size)
+        assert k >= its - 1
+        assert np.allclose(h[:k], hr[:k], rtol=1e-8, atol=1e-12 * np.linalg.norm(b)), np.max(np.abs(h[:k] - hr[:k]))
+        assert np.linalg.norm(x - xr) <= 1e-8 * np.linalg.norm(xr)
+
+
 def test_edge_cases(gpu_lib):
     A = matgen.poisson_2d(4, 4, 5.0)
     Ad = gpu.Device_matrix(A)
