@@ -854,6 +854,56 @@ ell_spmv_kernel(int nrow, long long ld, const int* __restrict__ col, const T* __
   }
 }
 
+// FP32: two rows a thread, so that a slot's columns and values come as 8-byte
+// loads; a row stops at its own length.  What bounds the FP32 rows is the
+// number of loads in flight, not the bytes: 131 x 113 x 97 grid, back to back,
+// 20.8 us one row a thread, 16.9 so (5 CTAs per SM: at 6 the registers spill,
+// 27.5).  `ld`, a multiple of 32, keeps the slots 8-byte aligned.
+template <class Epi, int U, int MINB>
+__global__ void __launch_bounds__(kThreads, MINB)
+ell_pair_kernel(int nrow, long long ld, const int* __restrict__ col, const float* __restrict__ va,
+                const int* __restrict__ rowlen, const float* __restrict__ x, Epi epi, RedWs ws, const Scalars* sc) {
+  constexpr int NR = Epi::kNR;
+  if (solve_done(sc)) return;
+  double red[NR > 0 ? NR : 1];
+#pragma unroll
+  for (int j = 0; j < (NR > 0 ? NR : 1); ++j) red[j] = 0.0;
+  for (int i = 2 * (blockIdx.x * kThreads + threadIdx.x); i < nrow; i += 2 * gridDim.x * kThreads) {
+    const int n0 = rowlen[i], n1 = i + 1 < nrow ? rowlen[i + 1] : 0;
+    const int n = max(n0, n1);
+    const int2* cp = reinterpret_cast<const int2*>(col + i);
+    const float2* vp = reinterpret_cast<const float2*>(va + i);
+    const long long step = ld / 2;
+    float s0 = 0.0f, s1 = 0.0f;
+    for (int k = 0; k < n; k += U) {
+      int2 c[U];
+      float2 v[U];
+      float x0[U], x1[U];
+#pragma unroll
+      for (int j = 0; j < U; ++j)
+        if (k + j < n) {
+          c[j] = __ldcs(cp + (k + j) * step);
+          v[j] = __ldcs(vp + (k + j) * step);
+        }
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        if (k + j < n0) x0[j] = __ldg(x + c[j].x);
+        if (k + j < n1) x1[j] = __ldg(x + c[j].y);
+      }
+#pragma unroll
+      for (int j = 0; j < U; ++j) {
+        if (k + j < n0) s0 = add(s0, mul(v[j].x, x0[j]));
+        if (k + j < n1) s1 = add(s1, mul(v[j].y, x1[j]));
+      }
+    }
+    reduce_terms<NR>(ws, i, red, [&](double* rr) { epi(i, s0, rr); });
+    if (i + 1 < nrow) reduce_terms<NR>(ws, i + 1, red, [&](double* rr) { epi(i + 1, s1, rr); });
+  }
+  if constexpr (NR > 0) {
+    grid_reduce<NR>(red, ws, [&](const double* t) { epi.finalize(t); });
+  }
+}
+
 // ------------------------------------------------------------------
 // Jagged diagonal: one thread per permuted position i, sweeping the
 // diagonals that reach it (coalesced across i), then y[perm[i]] = sum.
@@ -1141,11 +1191,16 @@ void launch_spmv(const sk_matrix_s* A, const T* x, Epi const& epi, RedWs ws,
       break;
     }
     case SK_ELL:
-      SK_LAUNCH((ell_spmv_kernel<T, Epi, 4, false, SpmvTune<T, Epi>::kMinB>),
-                row_grid<Epi>(A, A->nrow, SpmvTune<T, Epi>::kMinB), kThreads, 0, st,
-                static_cast<int>(A->nrow), static_cast<long long>(A->ell.ld), A->ell.col,
-                static_cast<const T*>(A->ell.vals),
-                A->ell.rowlen, x, epi, ws, sc);
+      if constexpr (sizeof(T) == 4)
+        SK_LAUNCH((ell_pair_kernel<Epi, 4, 5>), row_grid<Epi>(A, (A->nrow + 1) / 2, 5), kThreads, 0, st,
+                  static_cast<int>(A->nrow), static_cast<long long>(A->ell.ld), A->ell.col,
+                  static_cast<const float*>(A->ell.vals), A->ell.rowlen, x, epi, ws, sc);
+      else
+        SK_LAUNCH((ell_spmv_kernel<T, Epi, 4, false, SpmvTune<T, Epi>::kMinB>),
+                  row_grid<Epi>(A, A->nrow, SpmvTune<T, Epi>::kMinB), kThreads, 0, st,
+                  static_cast<int>(A->nrow), static_cast<long long>(A->ell.ld), A->ell.col,
+                  static_cast<const T*>(A->ell.vals),
+                  A->ell.rowlen, x, epi, ws, sc);
       break;
     case SK_JAD:
       SK_LAUNCH((jad_spmv_kernel<T, Epi, 4, false, SpmvTune<T, Epi>::kMinB>),

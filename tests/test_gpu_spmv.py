@@ -230,3 +230,26 @@ def test_panel_copy_only_where_the_order_is_not_kept(gpu_lib, oracle):
     assert Zd.add_panels() and Zd.layout() == "panels"
     x = matgen.uniform_vector(Z.shape()[0], seed=2)
     assert np.array_equal(gpu.multiply(Zd, x), oracle.spmv(Z, x))
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 31, 511, 512, 513, 2561])
+def test_ell_f32_two_rows_a_thread(gpu_lib, oracle, n):
+    """The FP32 ELLPACK product takes two rows a thread: an odd last row, rows
+    of unlike length in a pair (empty ones among them), more slots than a
+    round, and an x that starts off the 8-byte grid, bit for bit."""
+    import torch
+    rng = np.random.default_rng(n)
+    lens = rng.integers(0, 12, size=n)
+    lens[0] = min(n, 11)
+    rows = np.repeat(np.arange(n), np.minimum(lens, n))
+    A = formats.Compressed_row_matrix.from_entries((n, n), rows, rng.integers(0, n, rows.size),
+                                                   rng.standard_normal(rows.size), dtype=np.float32)
+    Ed = gpu.to_ellpack(gpu.Device_matrix(A))
+    x = matgen.uniform_vector(n, seed=2, dtype=np.float32)
+    buf = torch.empty(n + 1, dtype=torch.float32, device="cuda")
+    for shift in (0, 1):
+        xd = buf[shift:shift + n]
+        xd.copy_(torch.from_numpy(x))
+        yd = torch.full((n,), float("nan"), dtype=torch.float32, device="cuda")
+        Ed.spmv(xd, yd)
+        assert np.array_equal(yd.cpu().numpy(), oracle.spmv(A, x))
