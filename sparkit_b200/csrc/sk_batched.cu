@@ -51,9 +51,9 @@ struct sk_batch_s {
   int* cl_order = nullptr;  // per class: its systems, longest first, then the systems left to batched_cg_kernel
   std::vector<int> cl_first;            // first entry of each class in cl_order, and the end
   std::vector<std::vector<int>> cl_at;  // per class: its systems' positions in `order`, ascending
-  int cl_ctas[8] = {};  // per class: CTAs in flight
-  cudaStream_t fork[8] = {};
-  cudaEvent_t ev_fork = nullptr, ev_join[8] = {};
+  int cl_ctas[16] = {};  // per class: CTAs in flight
+  cudaStream_t fork[16] = {};
+  cudaEvent_t ev_fork = nullptr, ev_join[16] = {};
   // cached graph of the last solve
   cudaGraphExec_t graph = nullptr;
   const void* graph_key[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -625,8 +625,11 @@ const ClusterClass kClasses[] = {
     {1, 512, 5376, batched_cluster_kernel<1, 512, 2>},
     {1, 1024, 10848, batched_cluster_kernel<1, 1024, 1>},
     {2, 1024, 10848, batched_cluster_kernel<2, 1024, 1>},
+    {3, 1024, 10848, batched_cluster_kernel<3, 1024, 1>},
     {4, 1024, 10848, batched_cluster_kernel<4, 1024, 1>},
-    {8, 1024, 10848, batched_cluster_kernel<8, 1024, 1>},
+    {5, 1024, 10848, batched_cluster_kernel<5, 1024, 1>},
+    {6, 1024, 10848, batched_cluster_kernel<6, 1024, 1>},
+    {7, 1024, 10848, batched_cluster_kernel<7, 1024, 1>},
 };
 constexpr int kNumClasses = sizeof(kClasses) / sizeof(kClasses[0]);
 
@@ -756,7 +759,7 @@ sk_status enqueue_batch(sk_batch_s* B, const Variant& v, int ctas, BatchArgs a, 
     return static_cast<int>(std::lower_bound(at.begin(), at.end(), limit) - at.begin());
   };
   SK_CUDA(cudaEventRecord(B->ev_fork, st));
-  bool joined[8] = {};
+  bool joined[16] = {};
   for (int k = kNumClasses; k >= 0; --k) {
     const int count = taken(k);
     if (!count) continue;

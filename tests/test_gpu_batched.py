@@ -72,7 +72,7 @@ def test_batch_rejects_coupled_systems(gpu_lib):
 
 
 def test_cluster_classes_and_their_edges(gpu_lib):
-    """One lane per row solves a system on a cluster of 1 to 8 CTAs by its
+    """One lane per row solves a system on a cluster of 1 to 7 CTAs by its
     size: systems at the classes' limits and one row beside them, with rows
     and slices that do not fill, an empty one, one whose columns are spread
     over the whole system (every gather crosses CTAs), and the two kinds that
@@ -86,8 +86,8 @@ def test_cluster_classes_and_their_edges(gpu_lib):
         return sp.diags([np.full(n - 1, -1.0), np.full(n, 2.5), np.full(n - 1, -1.0)], [-1, 0, 1]) if n > 1 else \
             sp.csr_matrix([[2.5]])
 
-    mats = [chain(n) for n in (1, 31, 32, 33, 1000, 5376, 5377, 10848, 10849, 21696, 21697, 43392, 43393, 65536,
-                               65537)]
+    mats = [chain(n) for n in (1, 31, 32, 33, 1000, 5376, 5377, 10848, 10849, 21696, 21697, 32544, 32545, 43392,
+                               43393, 54240, 54241, 65088, 65089, 65536, 65537)]
     g = matgen.laplacian_2d_dirichlet(171)
     L = sp.csr_matrix((g.values(), g.col_ind(), g.row_ptr()), g.shape()) + 0.1 * sp.identity(171 * 171)
     perm = rng.permutation(171 * 171)
