@@ -272,6 +272,7 @@ void destroy_handle(sk_matrix A) {
   for (void* p : A->allocations) cudaFree(p);
   if (A->io) cudaFree(A->io);
   if (A->pipe) destroy_host_pipe(A->pipe);
+  destroy_tiles(A);
   if (A->ws) cudaFree(A->ws);
   if (A->ws2) cudaFree(A->ws2);
   if (A->stream) cudaStreamDestroy(A->stream);
@@ -324,6 +325,21 @@ static sk_status build_sell(sk_matrix A, const int64_t* rp, cudaStream_t st_) {
   return SK_OK;
 }
 
+// A copy that a product can do without: where the device has no room for it,
+// what it took is given back and the handle stays as it was.
+template <class Build>
+static sk_status optional_copy(sk_matrix A, Build const& build) {
+  const size_t mark = A->allocations.size();
+  const i64 bytes = A->device_bytes;
+  const sk_status s = build();
+  if (s != SK_OUT_OF_MEMORY) return s;
+  cudaGetLastError();
+  for (size_t k = mark; k < A->allocations.size(); ++k) cudaFree(A->allocations[k]);
+  A->allocations.resize(mark);
+  A->device_bytes = bytes;
+  return SK_OK;
+}
+
 // The split product's row lists (long rows by decreasing length, ties in
 // row order; short rows in row order) for a CSR handle without SELL-32
 // whose rows longer than kHybLong hold at least half of the entries.  The
@@ -353,7 +369,7 @@ static sk_status build_hybrid(sk_matrix A, const int64_t* rp, cudaStream_t st_) 
   const double short_work = 2.0 * static_cast<double>(A->nnz - long_nnz);
   A->csr.hyb_long_frac = static_cast<double>(long_nnz) / (static_cast<double>(long_nnz) + short_work);
   A->csr.hyb = true;
-  return SK_OK;
+  return optional_copy(A, [&] { return build_tiles(A, long_nnz, rp[longs[0] + 1] - rp[longs[0]], st_); });
 }
 
 // Adds the sliced copy of a 2x2 or 3x3 BSR handle when every block row has
@@ -420,7 +436,7 @@ sk_status csr_finish(sk_matrix A, const int64_t* row_ptr, cudaStream_t st_) {
   if ((st = build_sell(A, row_ptr, st_)) != SK_OK) return st;
   if (!A->csr.sell) return build_hybrid(A, row_ptr, st_);
   SK_CUDA(cudaStreamSynchronize(st_));
-  return build_stencil(A);
+  return optional_copy(A, [&] { return build_stencil(A); });
 }
 
 }  // namespace sk

@@ -26,7 +26,12 @@ constexpr int kBsrTileVals = 4096;  // BSR: block values staged per CTA
 constexpr int kMaxRed = 4;       // fused reductions carried per kernel
 constexpr i64 kStencilMinEntries = 1 << 19;  // below, the products are bound by launch latency
 constexpr i64 kTileSmem = 192 * 1024;    // bytes of x in a CTA's shared memory
-constexpr i64 kTileMinEntries = 1 << 20;  // fewest entries of the long rows
+// Fewest entries of the long rows.  Split against tiles, Zipf(1.5) rows of
+// random columns: FP64 34 against 45 us at 5.4M entries, 71 against 60 at 10.9M,
+// 144 against 94 at 22M, 437 against 228 at 69M; FP32 (whose x is half as far
+// beyond L1) 41 against 54 at 10.9M, 92 against 79 at 22M, 301 against 182 at 69M.
+constexpr i64 kTileMinEntries64 = i64(8) << 20, kTileMinEntries32 = i64(16) << 20;
+constexpr i64 kTileSegment = 96;          // entries a long row should have in a panel
 constexpr int kSellMaxRow = 64;  // CSR rows up to this length use SELL-32
 constexpr int kDiaMax = 16;      // diagonals of the diagonal copy of a CSR handle
 constexpr int kPanelSmem = 220 * 1024;  // dynamic shared memory of a column-panel CTA (at most)
@@ -81,6 +86,13 @@ extern std::atomic<i64> g_launches;
 // Device layouts
 // ------------------------------------------------------------------
 
+// Orders the products of one handle that share its partial sums: a product
+// waits, on its stream, for the one before, whatever stream that ran on.
+struct TileLock {
+  std::mutex m;
+  cudaEvent_t used = nullptr;
+};
+
 // CSR: int32 indices; arrays padded by 4 entries so that the 16-byte
 // vector loads of a tile's last group stay inside the allocation.
 // part[nparts+1] are the first rows of the row blocks one CTA handles.
@@ -114,6 +126,22 @@ struct Csr {
   int* hyb_long = nullptr;
   int hyb_nshort = 0, hyb_nlong = 0;
   double hyb_long_frac = 0.0;
+  // Panel-major copy of the long rows (sk_tile.cu), beside the row lists.
+  // tl_part holds one product's partial sums; tl_lock orders the products
+  // of one handle that use it.
+  bool tile = false;
+  int tl_panels = 0, tl_width = 0;
+  int* tl_unit = nullptr;        // first slice of each CTA, and the end
+  int* tl_slices_of = nullptr;   // first slice of each panel, and the end
+  int* tl_off = nullptr;         // first entry of each slice
+  unsigned short* tl_len = nullptr;  // per slice and lane
+  int* tl_dst = nullptr;         // per slice and lane: the partial sum, or -1
+  unsigned short* tl_col = nullptr;  // column inside the panel
+  void* tl_vals = nullptr;
+  int* tl_row_first = nullptr;   // per long row: its first partial sum, and the end
+  void* tl_part = nullptr;
+  double tl_long_frac = 0.0;
+  TileLock* tl_lock = nullptr;
   // Column-panel copy (sk_matrix_add_panels, sk_panel.cu): every row summed
   // in the reference's order whatever its length.  The rows are cut into pn_blocks
   // row blocks of about equal entries, one CTA each; the columns into
@@ -418,7 +446,7 @@ sk_status build_dia_f32(sk_matrix A);
 sk_status build_panel(sk_matrix A, const int64_t* rp, cudaStream_t st);
 // The panel-major copy of the long rows of a split handle; a no-op when it
 // does not qualify.
-sk_status build_tiles(sk_matrix A, i64 long_nnz, cudaStream_t st);
+sk_status build_tiles(sk_matrix A, i64 long_nnz, i64 longest, cudaStream_t st);
 void destroy_tiles(sk_matrix A);
 // Whether a square CSR handle on these diagonals is symmetric bit for bit.
 sk_status csr_symmetric(sk_matrix A, std::vector<int> const& offsets, bool* sym);

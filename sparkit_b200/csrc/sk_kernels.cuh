@@ -415,11 +415,14 @@ sell_spmv_kernel(int nrow, const int* __restrict__ off, const unsigned char* __r
 // bits of sparse_blas.hpp:25-28).  No shared memory, so the L1 serves the
 // random gathers of x only.
 // ------------------------------------------------------------------
-template <typename T, class Epi, int MINB>
+// With TILE the long rows' entries were summed by tile_part_kernel and a long
+// row is the sum of its partial sums, taken the same way.
+template <typename T, class Epi, int MINB, bool TILE>
 __global__ void __launch_bounds__(kThreads, MINB)
 hyb_spmv_kernel(const int* __restrict__ rp, const int* __restrict__ ci, const T* __restrict__ va,
                 const T* __restrict__ x, const int* __restrict__ short_rows, int nshort,
-                const int* __restrict__ long_rows, int nlong, int long_ctas, Epi epi, RedWs ws,
+                const int* __restrict__ long_rows, int nlong, int long_ctas,
+                const int* __restrict__ part_first, const T* __restrict__ part, Epi epi, RedWs ws,
                 const Scalars* sc) {
   constexpr int NR = Epi::kNR;
   if (solve_done(sc)) return;
@@ -431,6 +434,26 @@ hyb_spmv_kernel(const int* __restrict__ rp, const int* __restrict__ ci, const T*
     constexpr int W = kThreads / 32;
     const int lane = threadIdx.x & 31;
     const int nw = long_ctas * W;
+    if constexpr (TILE) {  // eight lanes to a row, up to 64 partial sums in one round
+      const int l8 = lane & 7;
+      for (int w = ((static_cast<int>(blockIdx.x) - short_ctas) * kThreads + threadIdx.x) >> 3; w < nlong;
+           w += nw * 4) {
+        const int row = __ldg(long_rows + w);
+        const int b = __ldg(part_first + w), e = __ldg(part_first + w + 1);
+        T sum = T(0);
+        for (int k0 = b + l8; k0 < e; k0 += 64) {
+          T v[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[j] = k0 + 8 * j < e ? __ldcs(part + k0 + 8 * j) : T(0);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sum = add(sum, v[j]);
+        }
+        const unsigned grp = 0xffu << (lane & 24);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) sum = add(sum, __shfl_xor_sync(grp, sum, o));
+        if (l8 == 0) reduce_terms<NR>(ws, row, red, [&](double* rr) { epi(row, sum, rr); });
+      }
+    } else
     for (int w = (static_cast<int>(blockIdx.x) - short_ctas) * W + (threadIdx.x >> 5); w < nlong; w += nw) {
       const int row = __ldg(long_rows + w);
       const int b = __ldg(rp + row), e = __ldg(rp + row + 1);
@@ -464,6 +487,97 @@ hyb_spmv_kernel(const int* __restrict__ rp, const int* __restrict__ ci, const T*
   }
   if constexpr (NR > 0) {
     grid_reduce<NR>(red, ws, [&](const double* t) { epi.finalize(t); });
+  }
+}
+
+// ------------------------------------------------------------------
+// The long rows' partial sums over the panel-major copy (sk_tile.cu).  What
+// bounds hyb_spmv_kernel on a matrix of random columns is its gathers of x,
+// one L2 request each (1M rows, 65M entries in long rows: 433 us against the
+// 106 us that the matrix's bytes take).  Here each CTA, one to an SM, holds
+// the panel of x that its run of slices needs in shared memory and its 32
+// warps draw slices from a counter, the longest segments first; a lane sums
+// its segment entry after entry, eight values and columns in flight.
+// The whole product of that matrix (L2 cold): 459 us split, 259 so, of which 185 are
+// spent here (waiting for loads: 31 warps an SM, 24% of issue slots used) and
+// 60 on the other rows.  Rounds of 12 at 512 threads with the next round's
+// loads issued ahead were slower (362 in all).
+// ------------------------------------------------------------------
+constexpr int kTileThreads = 1024;
+
+template <typename T>
+struct TileArgs {
+  const int* unit;
+  const int* slices_of;
+  const int* off;
+  const unsigned short* len;
+  const int* dst;
+  const unsigned short* col;
+  const T* val;
+  const T* x;
+  T* part;
+  int panels, width, ncol;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(kTileThreads, 1) tile_part_kernel(TileArgs<T> a, const Scalars* sc) {
+  extern __shared__ __align__(16) unsigned char tile_smem[];
+  __shared__ int s_next;
+  T* xs = reinterpret_cast<T*>(tile_smem);
+  if (solve_done(sc)) return;
+  const int u0 = a.unit[blockIdx.x], u1 = a.unit[blockIdx.x + 1];
+  const int lane = threadIdx.x & 31;
+  for (int p = 0; p < a.panels; ++p) {
+    const int s0 = max(u0, a.slices_of[p]), s1 = min(u1, a.slices_of[p + 1]);
+    if (s0 >= s1) continue;
+    const int c0 = p * a.width, w = min(a.width, a.ncol - c0);
+    __syncthreads();  // the panel before is done with
+    if (threadIdx.x == 0) s_next = s0;
+#pragma unroll 8
+    for (int k = threadIdx.x; k < w; k += kTileThreads) xs[k] = __ldg(a.x + c0 + k);
+    __syncthreads();
+    // the next slice's place and lengths are on their way while one is summed
+    auto next = [&](int& s, int& n, int& dst, int& off) {
+      s = lane == 0 ? atomicAdd(&s_next, 1) : 0;
+      s = __shfl_sync(0xffffffffu, s, 0);
+      n = 0;
+      dst = -1;
+      off = 0;
+      if (s < s1) {
+        n = __ldcs(a.len + static_cast<long long>(s) * 32 + lane);
+        dst = __ldcs(a.dst + static_cast<long long>(s) * 32 + lane);
+        off = __ldg(a.off + s);
+      }
+    };
+    int s, n, dst, off;
+    next(s, n, dst, off);
+    while (s < s1) {
+      int s2, n2, dst2, off2;
+      next(s2, n2, dst2, off2);
+      const unsigned short* cp = a.col + off + lane;
+      const T* vp = a.val + off + lane;
+      T sum = T(0);
+      for (int k0 = 0; k0 < n; k0 += 8) {
+        T v[8];
+        int c[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          c[j] = 0;
+          if (k0 + j < n) {
+            v[j] = __ldcs(vp + 32 * (k0 + j));
+            c[j] = __ldcs(cp + 32 * (k0 + j));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (k0 + j < n) sum = add(sum, mul(v[j], xs[c[j]]));
+      }
+      if (dst >= 0) a.part[dst] = sum;
+      s = s2;
+      n = n2;
+      dst = dst2;
+      off = off2;
+    }
   }
 }
 
@@ -1120,6 +1234,17 @@ inline int row_grid(const sk_matrix_s* A, i64 rows, int minb) {
   return full < wave ? (full > 0 ? full : 1) : wave;
 }
 
+// Whether a product on this stream can use the handle's partial sums: not
+// while it is captured, since a replay would not wait for the others.
+inline bool tile_usable(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return cap == cudaStreamCaptureStatusNone;
+}
+
 // Launches y-epilogue SpMV on any format.  vals_override lets the
 // mixed-precision path run the FP32 copy of an FP64 CSR handle.
 template <typename T, class Epi>
@@ -1179,10 +1304,27 @@ void launch_spmv(const sk_matrix_s* A, const T* x, Epi const& epi, RedWs ws,
         constexpr int MB = 6;  // 40 registers: four loads and gathers in flight per lane without spills
         const int grid = A->sm_count * MB;
         const int nl = A->csr.hyb_nlong, ns = A->csr.hyb_nshort;
-        int lc = static_cast<int>(grid * A->csr.hyb_long_frac + 0.5);
+        const bool tile = A->csr.tile && !vals_override && tile_usable(st);
+        int lc = static_cast<int>(grid * (tile ? A->csr.tl_long_frac : A->csr.hyb_long_frac) + 0.5);
         lc = nl == 0 ? 0 : ns == 0 ? grid : (lc < 1 ? 1 : lc > grid - 1 ? grid - 1 : lc);
-        SK_LAUNCH((hyb_spmv_kernel<T, Epi, MB>), grid, kThreads, 0, st, A->csr.row_ptr, A->csr.col_ind, v, x,
-                  A->csr.hyb_short, ns, A->csr.hyb_long, nl, lc, epi, ws, sc);
+        if (tile) {
+          const auto& C = A->csr;
+          std::lock_guard<std::mutex> lock(C.tl_lock->m);
+          cudaStreamWaitEvent(st, C.tl_lock->used, 0);
+          SK_LAUNCH(tile_part_kernel<T>, A->sm_count, kTileThreads, C.tl_width * sizeof(T), st,
+                    TileArgs<T>{C.tl_unit, C.tl_slices_of, C.tl_off, C.tl_len, C.tl_dst, C.tl_col,
+                                static_cast<const T*>(C.tl_vals), x, static_cast<T*>(C.tl_part), C.tl_panels,
+                                C.tl_width, static_cast<int>(A->ncol)},
+                    sc);
+          SK_LAUNCH((hyb_spmv_kernel<T, Epi, MB, true>), grid, kThreads, 0, st, C.row_ptr, C.col_ind, v, x,
+                    C.hyb_short, ns, C.hyb_long, nl, lc, C.tl_row_first, static_cast<const T*>(C.tl_part), epi, ws,
+                    sc);
+          cudaEventRecord(C.tl_lock->used, st);
+          break;
+        }
+        SK_LAUNCH((hyb_spmv_kernel<T, Epi, MB, false>), grid, kThreads, 0, st, A->csr.row_ptr, A->csr.col_ind, v, x,
+                  A->csr.hyb_short, ns, A->csr.hyb_long, nl, lc, static_cast<const int*>(nullptr),
+                  static_cast<const T*>(nullptr), epi, ws, sc);
         break;
       }
       SK_LAUNCH((csr_spmv_kernel<T, Epi>), A->csr.nparts, kThreads, 0, st,
