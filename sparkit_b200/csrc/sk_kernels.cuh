@@ -913,7 +913,7 @@ stencil_spmv_kernel(StencilArgs g, const T* __restrict__ va, const T* __restrict
                     const Scalars* sc) {
   constexpr int NR = Epi::kNR;
   constexpr int NL = SYM ? ND / 2 : 0, NP = ND - NL;  // diagonals read at another row, planes stored
-  if (solve_done(sc)) return;
+  const bool done = solve_done(sc);  // known when the first row's loads are back
   double red[NR > 0 ? NR : 1];
 #pragma unroll
   for (int j = 0; j < (NR > 0 ? NR : 1); ++j) red[j] = 0.0;
@@ -929,12 +929,14 @@ stencil_spmv_kernel(StencilArgs g, const T* __restrict__ va, const T* __restrict
       v[d] = SYM ? __ldg(at) : __ldcs(at);
       xv[d] = __ldg(x + c);
     }
+    if (done) return;
     T sum = T(0);
 #pragma unroll
     for (int d = 0; d < ND; ++d)
       if ((m >> d) & 1u) sum = add(sum, mul(v[d], xv[d]));
     reduce_terms<NR>(ws, i, red, [&](double* rr) { epi(i, sum, rr); });
   }
+  if (done) return;
   if constexpr (NR > 0) {
     grid_reduce<NR>(red, ws, [&](const double* t) { epi.finalize(t); });
   }

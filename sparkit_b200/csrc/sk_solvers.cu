@@ -1163,26 +1163,43 @@ struct FgGivens {
   }
 };
 
-// back_substitute (:365-379).
+// back_substitute (:365-379): one thread, in the reference's order.  For
+// cycles of up to kFgLocal steps the CTA first brings the triangle and g to
+// shared memory, so that the thread's chain of nj^2 / 2 dependent steps waits
+// on no load (a 30-step cycle: 50 us from global memory, under 10 so).
 template <typename T>
-struct FgBackSub {
-  Scalars* sc;
-  FgSmall sm;
-  int m;
-  __device__ void operator()() const {
-    if (sc->beta0) return;
-    const int um1 = m + 1;
-    const int nj = static_cast<int>(sc->jfinal) + 1;
-    for (int ii = nj; ii > 0; --ii) {
-      const int i = ii - 1;
-      T yi = static_cast<T>(sm.g[i]);
+__global__ void __launch_bounds__(kThreads) fg_back_sub_kernel(const Scalars* sc, FgSmall sm, int m) {
+  __shared__ double s_h[kFgLocal * (kFgLocal + 1) / 2];
+  __shared__ double s_g[kFgLocal], s_y[kFgLocal];
+  if (sc->beta0) return;
+  const int um1 = m + 1;
+  const int nj = static_cast<int>(sc->jfinal) + 1;
+  const bool local = nj <= kFgLocal;
+  if (local) {
+    for (int k = threadIdx.x; k < nj * nj; k += kThreads) {
+      const int i = k % nj, c = k / nj;
+      if (i <= c) s_h[c * (c + 1) / 2 + i] = sm.H[i + c * um1];
+    }
+    for (int k = threadIdx.x; k < nj; k += kThreads) s_g[k] = sm.g[k];
+    __syncthreads();
+  }
+  if (threadIdx.x != 0) return;
+  for (int ii = nj; ii > 0; --ii) {
+    const int i = ii - 1;
+    T yi = static_cast<T>(local ? s_g[i] : sm.g[i]);
+    if (local) {
+      for (int k = i + 1; k < nj; ++k)
+        yi = sub(yi, mul(static_cast<T>(s_h[k * (k + 1) / 2 + i]), static_cast<T>(s_y[k])));
+      yi = dvd(yi, static_cast<T>(s_h[i * (i + 1) / 2 + i]));
+      s_y[i] = static_cast<double>(yi);
+    } else {
       for (int k = i + 1; k < nj; ++k)
         yi = sub(yi, mul(static_cast<T>(sm.H[i + k * um1]), static_cast<T>(sm.y[k])));
       yi = dvd(yi, static_cast<T>(sm.H[i + i * um1]));
-      sm.y[i] = static_cast<double>(yi);
     }
+    sm.y[i] = static_cast<double>(yi);
   }
-};
+}
 
 // update_solution (:382-394): x_i += sum_k Z_k[i] y_k, summed in k order.
 template <typename T>
@@ -1202,7 +1219,15 @@ struct OpFgUpdateX {
   __device__ In load(i64 i) const { return {x[i]}; }
   __device__ void apply(i64 i, In const& q, double*) const {
     T sum = T(0);
-    for (int k = 0; k < nj; ++k) sum = add(sum, mul(Z[k * ldz + i], static_cast<T>(y[k])));
+    int k = 0;
+    for (; k + 8 <= nj; k += 8) {  // eight columns' loads in flight
+      T z[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) z[u] = Z[(k + u) * ldz + i];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) sum = add(sum, mul(z[u], static_cast<T>(y[k + u])));
+    }
+    for (; k < nj; ++k) sum = add(sum, mul(Z[k * ldz + i], static_cast<T>(y[k])));
     x[i] = add(q.x, sum);
   }
   __device__ void finalize(const double*) const {}
@@ -1337,15 +1362,17 @@ static sk_status fgmres_solve(sk_matrix A, sk_precond M, const T* b, T* x,
     }
     g_launches.fetch_add(1, std::memory_order_relaxed);
     if (hess64)
-      scalar_kernel<<<1, 1, 0, q>>>(FgBackSub<double>{c.sc, sm, m});
+      fg_back_sub_kernel<double><<<1, kThreads, 0, q>>>(c.sc, sm, m);
     else
-      scalar_kernel<<<1, 1, 0, q>>>(FgBackSub<T>{c.sc, sm, m});
+      fg_back_sub_kernel<T><<<1, kThreads, 0, q>>>(c.sc, sm, m);
     launch_vec(n, OpFgUpdateX<T>{x, Z, ldv, sm.y, 0}, c.ws, c.sc, q);
   };
   // Solves expected to run several cycles replay each cycle as a CUDA graph
-  // (one launch per cycle instead of ~m^2 / 2), captured on a created stream
-  // (the legacy stream cannot be captured; the caller's stream is drained
-  // first and this call returns after its last host read).
+  // (a cooperative launch costs the host more than a step of a small system
+  // the device), captured on a created stream (the legacy stream cannot be
+  // captured; the caller's stream is drained first and this call returns after
+  // its last host read).  In graphs of six steps, the later ones captured
+  // while the first ran, solves were 1 to 2.5% slower.
   const bool graphs = cfg->max_iterations >= 3 * static_cast<i64>(m) && n >= 1;
   cudaStream_t gs = st;
   if (graphs && (st == nullptr || st == cudaStreamLegacy || st == cudaStreamPerThread)) {

@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kThreads) restrict_kernel(int nx, int agg, int
                                                             const double* __restrict__ t, double* __restrict__ rc,
                                                             const Scalars* sc) {
   constexpr int kW = kThreads / 32;
-  if (solve_done(sc)) return;
+  const bool done = solve_done(sc);  // known when the cells are back
   const int I = blockIdx.x * kW + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (I >= nc) return;
@@ -110,7 +110,14 @@ __global__ void __launch_bounds__(kThreads) restrict_kernel(int nx, int agg, int
       if (c < cells) v[w] += t[static_cast<i64>(Y0 + c / agg) * nx + X0 + c % agg];
     }
   }
-  warp_reduce<kW>(v);
+  if (done) return;
+#pragma unroll
+  for (int w = 0; w < kW; ++w)
+    if (32 * w < cells) {  // the warps beyond hold zeros
+      double y[1] = {v[w]};
+      warp_reduce<1>(y);
+      v[w] = y[0];
+    }
   double x[1] = {0.0};
 #pragma unroll
   for (int w = 0; w < kW; ++w)
@@ -119,47 +126,70 @@ __global__ void __launch_bounds__(kThreads) restrict_kernel(int nx, int agg, int
   if (lane == 0) rc[I] = x[0];
 }
 
-// zc = Ainv rc: one warp per coarse row, lane-strided partial sums and a
-// shuffle tree.  The inverse is stored in FP32 (64 MiB at nc = 4096: half
+// zc = Ainv rc: column-strided partial sums and a shuffle tree, the eight
+// warps' sums in warp order.  The inverse is stored in FP32 (64 MiB at nc = 4096: half
 // the bytes of the FP64 inverse, and within the L2) and every product is
 // formed and summed in FP64; the float rounding of the inverse (relative
 // 6e-8 per entry) perturbs the coarse correction of a preconditioner only.
-// Each lane reads four consecutive floats (16 bytes) per step, four steps'
-// loads in flight before their products are summed (in step order).
-__global__ void __launch_bounds__(kThreads) coarse_gemv_kernel(int nc, const float* __restrict__ ainv,
-                                                               const double* __restrict__ rc,
-                                                               double* __restrict__ zc, const Scalars* sc) {
-  if (solve_done(sc)) return;
-  const int I = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (I >= nc) return;
-  const float* row = ainv + static_cast<i64>(I) * nc;
-  double s[1] = {0.0};
-  int j = 4 * lane;
+// The bytes of the inverse bound it.  A CTA takes kGemvRows rows and its eight
+// warps the columns, 128 at a time: a lane holds the entries of rc that it
+// needs in registers for all the rows, and all its 16-byte loads of four such
+// steps (at nc = 4096 all there are) are issued before anything is waited for,
+// the solve's flag included.  At nc = 4096 inside a solve, with
+// the inverse partly in L2: 15 us; 17 with one step's loads in flight, 25 with
+// a row to a warp (which reads rc once per row).
+constexpr int kGemvRows = 4, kGemvSteps = 4;
+__global__ void __launch_bounds__(kThreads, 2) coarse_gemv_kernel(int nc, const float* __restrict__ ainv,
+                                                                  const double* __restrict__ rc,
+                                                                  double* __restrict__ zc, const Scalars* sc) {
+  constexpr int R = kGemvRows, U = kGemvSteps, W = kThreads / 32;
+  __shared__ double part[W][R];
+  const bool done = solve_done(sc);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int I0 = blockIdx.x * R;
+  double s[R];
+#pragma unroll
+  for (int q = 0; q < R; ++q) s[q] = 0.0;
   if ((nc & 3) == 0) {
-    for (; j < nc; j += 512) {
-      float4 a[4];
-      double r[4][4];
+    for (int j0 = warp * 128 + 4 * lane; j0 < nc; j0 += U * W * 128) {
+      float4 a[U][R];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int jj = j + 128 * u;
-        if (jj < nc) {
-          a[u] = __ldg(reinterpret_cast<const float4*>(row + jj));
+      for (int u = 0; u < U; ++u)
 #pragma unroll
-          for (int k = 0; k < 4; ++k) r[u][k] = rc[jj + k];
-        }
+        for (int q = 0; q < R; ++q)
+          if (I0 + q < nc && j0 + u * W * 128 < nc)
+            a[u][q] = __ldg(reinterpret_cast<const float4*>(ainv + static_cast<i64>(I0 + q) * nc + j0 + u * W * 128));
+      if (done) break;
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int j = j0 + u * W * 128;
+        if (j >= nc) break;
+        const double2 lo = *reinterpret_cast<const double2*>(rc + j), hi = *reinterpret_cast<const double2*>(rc + j + 2);
+#pragma unroll
+        for (int q = 0; q < R; ++q)
+          if (I0 + q < nc)
+            s[q] += static_cast<double>(a[u][q].x) * lo.x + static_cast<double>(a[u][q].y) * lo.y +
+                    static_cast<double>(a[u][q].z) * hi.x + static_cast<double>(a[u][q].w) * hi.y;
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (j + 128 * u < nc)
-          s[0] += static_cast<double>(a[u].x) * r[u][0] + static_cast<double>(a[u].y) * r[u][1] +
-                  static_cast<double>(a[u].z) * r[u][2] + static_cast<double>(a[u].w) * r[u][3];
     }
   } else {
-    for (j = lane; j < nc; j += 32) s[0] += static_cast<double>(row[j]) * rc[j];
+    for (int j = threadIdx.x; j < nc; j += kThreads)
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        if (I0 + q < nc) s[q] += static_cast<double>(ainv[static_cast<i64>(I0 + q) * nc + j]) * rc[j];
   }
-  warp_reduce<1>(s);
-  if (lane == 0) zc[I] = s[0];
+  if (done) return;  // the same flag for every thread
+  warp_reduce<R>(s);
+  if (lane == 0)
+#pragma unroll
+    for (int q = 0; q < R; ++q) part[warp][q] = s[q];
+  __syncthreads();
+  if (threadIdx.x < R && I0 + threadIdx.x < nc) {
+    double t = 0.0;
+#pragma unroll
+    for (int w = 0; w < W; ++w) t += part[w][threadIdx.x];
+    zc[I0 + threadIdx.x] = t;
+  }
 }
 
 // z += P zc, z = P zc (set), or z += add (the smoother's share)
@@ -169,9 +199,10 @@ __global__ void __launch_bounds__(kThreads) prolong_kernel(i64 n, int nx, int ag
   if (solve_done(sc)) return;
   for (i64 i = blockIdx.x * static_cast<i64>(kThreads) + threadIdx.x; i < n;
        i += static_cast<i64>(gridDim.x) * kThreads) {
-    const int y = static_cast<int>(i / nx), x = static_cast<int>(i % nx);
+    const unsigned y = static_cast<unsigned>(i) / static_cast<unsigned>(nx);  // n < 2^31: a 32-bit division
+    const unsigned x = static_cast<unsigned>(i) - y * static_cast<unsigned>(nx);
     if (zc) {
-      const double c = zc[(y / agg) * mcx + x / agg];
+      const double c = zc[(y / static_cast<unsigned>(agg)) * mcx + x / static_cast<unsigned>(agg)];
       z[i] = set ? c : __dadd_rn(z[i], c);
     } else {
       z[i] = __dadd_rn(z[i], add[i]);
@@ -239,7 +270,7 @@ void twolevel_apply(const sk_precond_s* M, const double* r, double* z, RedWs ws,
   const sk_precond_s* S = M->smoother;
   auto coarse = [&](const double* t, int set) {  // z (+)= P Ac^-1 P^T t
     SK_LAUNCH(restrict_kernel, ceil_div(nc, kThreads / 32), kThreads, 0, st, nx, agg, mcx, nc, t, M->rc, sc);
-    SK_LAUNCH(coarse_gemv_kernel, ceil_div(nc, kThreads / 32), kThreads, 0, st, nc,
+    SK_LAUNCH(coarse_gemv_kernel, ceil_div(nc, kGemvRows), kThreads, 0, st, nc,
               M->coarse_inv, M->rc, M->zc, sc);
     SK_LAUNCH(prolong_kernel, ew_blocks(n), kThreads, 0, st, n, nx, agg, mcx, M->zc, nullptr, set, z, sc);
   };

@@ -89,3 +89,26 @@ def test_twolevel_rejects_bad_arguments(gpu_lib):
         gpu.twolevel(Ad, J, 32, 16, 4)  # 32 x 16 is not the matrix size
     with pytest.raises(_lib.SkError):
         gpu.twolevel(Ad, J, 32, 32, 0)
+
+
+@pytest.mark.parametrize("nx,ny,agg", [(8, 8, 8), (24, 40, 8), (48, 44, 4), (128, 66, 2), (128, 128, 2)])
+def test_coarse_product_sizes(gpu_lib, nx, ny, agg):
+    """Coarse systems of 1, 15, 132, 2112 and 4096 rows: one, an odd number,
+    part of a step, part of a round, and the most there may be.  The FP32
+    inverse is off by at most 2^-24 of each entry; twice that, entry by entry,
+    plus 1e-9 of the result for the FP64 parts."""
+    import torch
+    from tests.test_gpu_learned import rect_convdiff
+    A = rect_convdiff(nx, ny, 4)
+    M, P, Aci = _dense_parts(A, nx, ny, agg)
+    Ad = gpu.Device_matrix(A)
+    J = gpu.jacobi(Ad)
+    T = gpu.twolevel(Ad, J, nx, ny, agg)
+    r = np.random.default_rng(3).standard_normal(nx * ny)
+    rd = torch.from_numpy(r).cuda()
+    zd = torch.zeros_like(rd)
+    T.apply(rd, zd)
+    rc = P.T @ (r - M @ (r / M.diagonal()))
+    z = r / M.diagonal() + P @ (Aci @ rc)
+    bar = 2.0 ** -23 * (P @ (np.abs(Aci) @ np.abs(rc))) + 1e-9 * np.max(np.abs(z))
+    assert np.all(np.abs(zd.cpu().numpy() - z) <= bar)
