@@ -5,9 +5,11 @@ Headline: SpMV HBM GB/s, CSR FP64, 3-D 7-point Dirichlet Laplacian on a
 128^3 grid (n = 2,097,152, nnz = 14,581,760), the SpMV format-sweep
 configuration.  A step is one product y = A x.
 
-  value     algorithmic bytes of one product / device time per step
-            (CUDA events on the launching stream, inputs resident in HBM;
-            the matrix, x and y are 217 MB, above the 126 MB L2)
+  value     bytes of one product in the CSR format (217 MB: each array once)
+            / device time per step (CUDA events on the launching stream,
+            inputs resident in HBM, as many operand sets in turn as exceed
+            the 126 MB L2).  The device layout may move fewer bytes: the
+            roofline is that of the bytes moved
   e2e       the same metric through the drop-in call sk_spmv_host, with x
             copied in from pinned host memory and y copied back every step
   roofline  dominant kernel vs the measured HBM copy bandwidth
@@ -249,6 +251,30 @@ def time_device(fn, steps, warmup, stream):
     return e0.elapsed_time(e1) / steps  # ms per step
 
 
+def layout_bytes(Ad, dtype):
+    """Bytes of one product on the layout the handle runs on: of the stencil
+    copy of a symmetric 7-point matrix 4 planes, the row masks, x and y; else
+    the handle's own byte model."""
+    info = Ad.info()
+    if Ad.layout() == "stencil":
+        return info["nrow"] * (6 * np.dtype(dtype).itemsize + 2)
+    return info["spmv_bytes"]
+
+
+def rotate(make, bytes_one, total=300e6):
+    """Enough copies of a product's operands that one round of them exceeds
+    the 126 MB L2, and the call that steps through them."""
+    copies = [make() for _ in range(max(1, int(-(-total // bytes_one))) if bytes_one < 126e6 else 1)]
+    at = [0]
+
+    def step():
+        A, x, y, sptr = copies[at[0]]
+        at[0] = (at[0] + 1) % len(copies)
+        A.spmv(x, y, stream=sptr)
+
+    return step, copies
+
+
 def sweep(stream, grid):
     """GB/s of each format and precision (algorithmic bytes / event time)."""
     import torch
@@ -270,13 +296,18 @@ def sweep(stream, grid):
             Ad = gpu.Device_matrix(M)
             if fmt == "csr_diagonal_copy":
                 assert Ad.add_diagonals()
-            ms = time_device(lambda: Ad.spmv(xd, yd, stream=sptr), 300, 20, stream)
-            # spmv_bytes is the byte model of the layout the product reads
-            # (for the diagonal copy: its values and row masks, x and y)
+            step, copies = rotate(lambda: (gpu.Device_matrix(M), xd.clone(), yd.clone(), sptr), layout_bytes(Ad, dt))
+            ms = time_device(step, 300, 20, stream)
+            # spmv_bytes is the byte model of the format (for the diagonal
+            # copy: its values and row masks, x and y), layout_bytes that of
+            # the copy the product runs on
             info = Ad.info()
             out[f"lap3d_{fmt}_{tag}"] = {"gbs": info["spmv_bytes"] / ms / 1e6, "us": ms * 1e3,
                                          "bytes": info["spmv_bytes"], "layout": Ad.layout(),
+                                         "layout_bytes": layout_bytes(Ad, dt),
                                          "device_bytes": info["device_bytes"]}
+            for c in copies:
+                c[0].close()
             Ad.close()
     del A
     B = matgen.vector_laplacian_3d_bsr(grid, seed=1)
@@ -1202,10 +1233,8 @@ def main():
     info = Ad.info()
     bytes_one = info["spmv_bytes"]
     xd = torch.from_numpy(x).cuda()
-    yd = torch.empty_like(xd)
-
-    def step():
-        Ad.spmv(xd, yd, stream=sptr)
+    moved = layout_bytes(Ad, np.float64)
+    step, copies = rotate(lambda: (gpu.Device_matrix(A), xd.clone(), torch.empty_like(xd), sptr), moved)
 
     try:
         uuid = str(torch.cuda.get_device_properties(dev).uuid)
@@ -1270,13 +1299,20 @@ def main():
     assert np.isfinite(y_host).all()
 
     peak, peak_kind = measured_peak()
-    achieved = bytes_one / (ms * 1e-3) / 1e9
+    # the roofline is that of the bytes the product moves; `value` keeps the
+    # format's byte model, which a smaller device layout may exceed the peak of
+    achieved = moved / (ms * 1e-3) / 1e9
+    stencil = Ad.layout() == "stencil"
+    layout = Ad.layout()
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "peak_source": f"{peak_kind} (MEASURED_PEAKS.json hbm_gbs)" if peak_kind == "measured"
                 else "fallback 6650 GB/s",
-                "traffic": profiled_traffic("csr_spmv_f64_lap3d128"),
-                "kernel": "sell_spmv_kernel<double, EpiStore<double>, 4, false, 8>",
-                "bytes_model": "8*nnz + 4*nnz + 4*(n+1) + 8*n (x) + 8*n (y)", "bytes_per_launch": bytes_one}
+                "traffic": profiled_traffic("stencil_spmv_f64_lap3d128" if stencil else "csr_spmv_f64_lap3d128"),
+                "kernel": "stencil_spmv_kernel<double, EpiStore<double>, 7, true>" if stencil
+                else "sell_spmv_kernel<double, EpiStore<double>, 4, false, 8>",
+                "bytes_model": "4 planes of 8*n, 2*n (row masks), 8*n (x), 8*n (y)" if stencil
+                else "8*nnz + 4*nnz + 4*(n+1) + 8*n (x) + 8*n (y)", "bytes_per_launch": moved,
+                "format_bytes_per_launch": bytes_one}
 
     extra = {}
     if rank == 0 and world == 1 and not args.no_cpu:
@@ -1303,7 +1339,9 @@ def main():
             "vs_baseline": None, "dtype": "f64",
             "data": "synthetic (seeded 7-point Dirichlet Laplacian, x ~ U[-1,1] seed 1)",
             "config": {"workload": WORKLOAD, "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
-                       "l2": f"inputs {bytes_one / 1e6:.0f} MB per product > 126 MB L2, no flush"},
+                       "layout": layout,
+                       "l2": f"{moved / 1e6:.0f} MB per product, {len(copies)} operand sets in turn > 126 MB L2, "
+                             "no flush"},
             "e2e": {"value": bytes_one * world / e2e_s / 1e9, "unit": "GB/s",
                     "h2d_bytes_per_step": 8 * n, "d2h_bytes_per_step": 8 * n,
                     "ms_per_step": e2e_s * 1e3, "call": "sk_spmv_host (pinned host x, y)"},

@@ -329,8 +329,11 @@ __global__ void __launch_bounds__(NT, 1024 / NT) batched_cg_kernel(BatchView bv,
 // Row sums have the bits of batched_cg_kernel<1, NT> (FP32, storage order);
 // the dot products' partial sums meet in another order.
 //
-// 1024 systems of 1k to 64k rows (2-D and 3-D grids, sizes log-uniform): 105 ms with one CTA per system, 18.1 ms so.  Systems of more than
-// 65,536 rows (16-bit columns) or rows of more than 64 entries stay with
+// 1024 systems of 1k to 64k rows (2-D and 3-D grids, sizes log-uniform):
+// 105 ms with one CTA per system, 17.4 ms so (18.3 with clusters of 1, 2, 4 and
+// 8 only: those of 8 fit 120 SMs).  Two or four rows' entries in flight per
+// thread at 512 threads were slower (21 ms).  Systems of more than 65,536 rows
+// (16-bit columns) or rows of more than 64 entries stay with
 // batched_cg_kernel, as do two or more lanes per row.
 // ------------------------------------------------------------------
 struct ClusterView {

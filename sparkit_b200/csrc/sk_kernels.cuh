@@ -498,7 +498,7 @@ hyb_spmv_kernel(const int* __restrict__ rp, const int* __restrict__ ci, const T*
 // the panel of x that its run of slices needs in shared memory and its 32
 // warps draw slices from a counter, the longest segments first; a lane sums
 // its segment entry after entry, eight values and columns in flight.
-// The whole product of that matrix (L2 cold): 459 us split, 259 so, of which 185 are
+// The whole product, three such matrices in turn: 449 us split, 256 so, of which 185 are
 // spent here (waiting for loads: 31 warps an SM, 24% of issue slots used) and
 // 60 on the other rows.  Rounds of 12 at 512 threads with the next round's
 // loads issued ahead were slower (362 in all).
