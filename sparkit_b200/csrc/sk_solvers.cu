@@ -323,9 +323,8 @@ struct OpCgUpdate {
   double* hist;
   T alpha;
   __device__ bool prepare(const Scalars* s) {
-    if (solve_done(s)) return false;
-    alpha = static_cast<T>(s->alpha);
-    return true;
+    alpha = static_cast<T>(s->alpha);  // on its way together with the flag
+    return !solve_done(s);
   }
   struct In { T x, h, r, q, d; };
   __device__ In load(i64 i) const {
@@ -339,15 +338,24 @@ struct OpCgUpdate {
     if constexpr (LK == PK_JACOBI) red[1] += static_cast<double>(mul(ri, mul(v.d, ri)));
   }
   __device__ void finalize(const double* t) const {
-    sc->iters += 1;
+    // everything read in one batch: this thread's chain is what the next
+    // kernel waits for
+    const double bnorm = sc->bnorm, tol = sc->tol, rz = sc->rz;
+    const long long iters = sc->iters + 1, max_iters = sc->max_iters, len = sc->hist_len;
+    const int hist_on = sc->hist_on;
     const T rn = sqrt(static_cast<T>(t[0]));
-    record(sc, hist, static_cast<double>(rn));
-    const bool conv = rn / static_cast<T>(sc->bnorm) < static_cast<T>(sc->tol);
+    const bool conv = rn / static_cast<T>(bnorm) < static_cast<T>(tol);
+    sc->iters = iters;
+    sc->rnorm = static_cast<double>(rn);
+    if (hist_on) {
+      hist[len] = static_cast<double>(rn);
+      sc->hist_len = len + 1;
+    }
     sc->converged = conv ? 1 : 0;
-    if (conv || sc->iters >= sc->max_iters) sc->done = 1;
+    if (conv || iters >= max_iters) sc->done = 1;
     if (LK != PK_OTHER && !conv) {
       const T rz_new = static_cast<T>(LK == PK_JACOBI ? t[1] : t[0]);
-      sc->beta = static_cast<double>(rz_new / static_cast<T>(sc->rz));
+      sc->beta = static_cast<double>(rz_new / static_cast<T>(rz));
       sc->rz = static_cast<double>(rz_new);
     }
   }
@@ -382,9 +390,8 @@ struct OpCgDirection {
   const T* inv_d;
   T beta;
   __device__ bool prepare(const Scalars* s) {
-    if (solve_done(s)) return false;
-    beta = static_cast<T>(s->beta);
-    return true;
+    beta = static_cast<T>(s->beta);  // on its way together with the flag
+    return !solve_done(s);
   }
   struct In { T z, p; };
   __device__ In load(i64 i) const {
