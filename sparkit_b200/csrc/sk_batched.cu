@@ -437,6 +437,10 @@ __global__ void __launch_bounds__(NT, MINB) batched_cluster_kernel(ClusterView c
   if constexpr (C > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const unsigned p_addr = cl_smem(p);
   int set = 0;
+  // A CTA's shared memory may be written from outside only once it runs, and
+  // being placed together does not say that it does: without this barrier the
+  // first store below could come before the CTA that it goes to.
+  if constexpr (C > 1) cl_barrier<C>();
   for (int turn = 0;; turn ^= 1) {
     if (rank == 0 && tid == 0) {
       const int t = atomicAdd(counter, 1);

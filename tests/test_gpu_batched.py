@@ -120,3 +120,40 @@ def test_cluster_classes_and_their_edges(gpu_lib):
         for s in range(len(mats)):
             a, e = offs[s], offs[s + 1]
             assert np.linalg.norm(r[a:e]) <= 1.0001e-10 * np.linalg.norm(b[a:e]), (s, e - a)
+
+
+def chains(sizes, seed):
+    """Tridiagonal SPD systems of these sizes as one batch, and a right-hand side."""
+    offs = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    total = int(offs[-1])
+    i = np.arange(total)
+    cols = np.stack([i - 1, i, i + 1], 1)
+    keep = np.ones((total, 3), bool)
+    keep[offs[:-1], 0] = False
+    keep[offs[1:] - 1, 2] = False
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))])
+    va = np.tile(np.float32([-1.0, 2.5, -1.0]), (total, 1))[keep]
+    return offs, rp, cols[keep], va, np.random.default_rng(seed).uniform(-1, 1, total)
+
+
+def test_clusters_start_beside_other_work(gpu_lib):
+    """The CTAs of a cluster start one after another where other work holds
+    SMs: every solve of systems on clusters of 2 to 7 CTAs gives the same bits,
+    and the systems are solved."""
+    import torch
+    offs, rp, ci, va, b = chains([11000, 22000, 33000, 44000, 55000, 65200] * 8, seed=3)
+    B = gpu.Batch(offs, rp, ci, va)
+    bd = torch.from_numpy(b).cuda()
+    xd = torch.zeros_like(bd)
+    _, _, rel, conv = B.solve(bd, xd)
+    first = xd.clone()
+    assert conv.all() and (rel < 1e-10).all()
+    other, m = torch.cuda.Stream(), torch.randn(2048, 2048, device="cuda")
+    for _ in range(20):
+        xd.zero_()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(other):
+            for _ in range(20):
+                m = torch.tanh(m @ m)
+        _, _, rel, conv = B.solve(bd, xd)
+        assert conv.all() and torch.equal(xd, first)
