@@ -56,7 +56,7 @@ struct sk_batch_s {
   cudaEvent_t ev_fork = nullptr, ev_join[16] = {};
   // cached graph of the last solve
   cudaGraphExec_t graph = nullptr;
-  const void* graph_key[4] = {nullptr, nullptr, nullptr, nullptr};
+  const void* graph_key[7] = {};  // every pointer that its kernels hold
   int graph_variant = -1;
   int graph_ctas = 0;
   sk::i64 graph_launches = 0;
@@ -999,9 +999,10 @@ SK_API sk_status sk_batched_cg_solve(sk_batch B, const double* b_dev, double* x_
   SK_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(s)));
   // The launch (queue reset + persistent kernel) is captured once into a
   // CUDA graph and replayed while the pointers and settings stay the same.
-  const void* key[4] = {b_dev, x_dev, res->inner_iterations, B->ws};
+  const void* key[7] = {b_dev, x_dev, B->ws, res->inner_iterations, res->outer_iterations, res->relative_residual,
+                        res->converged};
   const bool same = B->graph && B->graph_variant == vi && B->graph_ctas == ctas &&
-                    std::equal(key, key + 4, B->graph_key) &&
+                    std::equal(key, key + 7, B->graph_key) &&
                     std::memcmp(&B->graph_cfg, cfg, sizeof(*cfg)) == 0;
   if (!same) {
     if (B->graph) {
@@ -1020,7 +1021,7 @@ SK_API sk_status sk_batched_cg_solve(sk_batch B, const double* b_dev, double* x_
     if (g) cudaGraphDestroy(g);
     if (st != SK_OK) return st;
     if (e != cudaSuccess) return cuda_fail(e, "batched solve capture");
-    std::copy(key, key + 4, B->graph_key);
+    std::copy(key, key + 7, B->graph_key);
     B->graph_variant = vi;
     B->graph_ctas = ctas;
     B->graph_cfg = *cfg;

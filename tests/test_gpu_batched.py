@@ -157,3 +157,36 @@ def test_clusters_start_beside_other_work(gpu_lib):
                 m = torch.tanh(m @ m)
         _, _, rel, conv = B.solve(bd, xd)
         assert conv.all() and torch.equal(xd, first)
+
+
+@pytest.mark.parametrize("changed", range(4))
+def test_results_go_to_the_arrays_of_the_call(gpu_lib, changed):
+    """Another array for any one of the four results: this call writes to it, and
+    to the former one no more."""
+    import ctypes
+
+    import torch
+    offs, rp, ci, va, b = chains([100, 700, 12000], seed=5)
+    B = gpu.Batch(offs, rp, ci, va)
+    bd = torch.from_numpy(b).cuda()
+    xd = torch.zeros_like(bd)
+    L, cfg = _lib.lib(), B._cfg(gpu.Batch_config())
+
+    def solve(arrays):
+        xd.zero_()
+        torch.cuda.synchronize()
+        res = _lib.BatchResults(*[ctypes.c_void_p(a.data_ptr()) for a in arrays])
+        _lib.check(L.sk_batched_cg_solve(B.handle, ctypes.c_void_p(bd.data_ptr()), ctypes.c_void_p(xd.data_ptr()),
+                                         ctypes.byref(cfg), ctypes.byref(res), None))
+
+    types = [torch.int32, torch.int32, torch.float64, torch.int32]
+    old = [torch.full((3,), -1, dtype=t, device="cuda") for t in types]
+    solve(old)
+    want = [a.clone() for a in old]
+    new = list(old)
+    new[changed] = torch.full_like(old[changed], -1)
+    old[changed].fill_(-7)
+    solve(new)
+    for a, w in zip(new, want):
+        assert torch.equal(a, w)
+    assert (old[changed] == -7).all()
