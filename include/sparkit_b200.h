@@ -613,7 +613,7 @@ typedef struct {
   int64_t max_inner;
   int32_t adaptive_last_step;
   int32_t lanes_per_row;     /* 1, 2, 4 or 8 (from sk_batched_autotune) */
-  int32_t threads_per_cta;   /* 256, 512 or 1024 */
+  int32_t threads_per_cta;   /* 256, 512 or 1024; see sk_batched_cg_solve */
 } sk_batch_config;
 
 /* Device arrays of nsys entries each, written by the solve. */
@@ -624,19 +624,25 @@ typedef struct {
   int32_t* converged;
 } sk_batch_results;
 
-/* Solves every system in one persistent launch (FP32 Jacobi-CG inside FP64
- * iterative refinement, conjugate_gradient.hpp:122-312 per system), one CTA
- * per system at a time taken from a longest-first queue.  The launch is
- * captured into a CUDA graph and replayed while the pointers and settings
- * stay the same.  b and x are FP64 device vectors over all rows; x holds the
- * initial guesses and receives the solutions. */
+/* Solves every system (FP32 Jacobi-CG inside FP64 iterative refinement,
+ * conjugate_gradient.hpp:122-312 per system).  With lanes_per_row = 1 a system
+ * of at most 65,536 rows of at most 64 entries runs on a thread-block cluster
+ * of 1 to 7 CTAs by its size, one launch per cluster size side by side, and
+ * threads_per_cta does not apply to it; all other systems, and all of them with
+ * more lanes, share one launch of one CTA per system at a time.  Each launch
+ * takes its systems from a longest-first queue.  The launches are
+ * captured into a CUDA graph and replayed while the pointers (of the results
+ * too) and settings stay the same.  b and x are FP64 device vectors over all
+ * rows; x holds the initial guesses and receives the solutions. */
 SK_API sk_status sk_batched_cg_solve(sk_batch B, const double* b_dev,
                                      double* x_dev, const sk_batch_config* cfg,
                                      sk_batch_results* res, sk_stream s);
 
 /* Times every (lanes_per_row, threads_per_cta) variant on the `sample`
  * largest systems and returns the fastest; ms_out (may be NULL) receives
- * sk_batched_variant_count() timings.  x is overwritten with zeros. */
+ * sk_batched_variant_count() timings.  Where threads_per_cta applies to none of
+ * the sampled systems, the one-lane variants are one and are timed once.  x is
+ * overwritten with zeros. */
 SK_API sk_status sk_batched_autotune(sk_batch B, const double* b_dev,
                                      double* x_dev, const sk_batch_config* cfg,
                                      sk_batch_results* res, int64_t sample,

@@ -1,23 +1,30 @@
-// sk_batched.cu -- thousands of independent SPD systems solved in one
-// persistent launch: conjugate gradient (conjugate_gradient.hpp:122-312,
-// Jacobi-preconditioned, FP32 values and vectors) inside FP64 iterative
-// refinement, one CTA per system at a time.
+// sk_batched.cu -- thousands of independent SPD systems solved in one call:
+// conjugate gradient (conjugate_gradient.hpp:122-312, Jacobi-preconditioned,
+// FP32 values and vectors) inside FP64 iterative refinement.
 //
 // No reference counterpart: the reference solves one system per call; the
 // comparison point is a loop of the plain solver over the systems.
 //
 // Layout: the systems are the diagonal blocks of one block-diagonal CSR
 // matrix (global row numbering, FP32 values); system s owns rows
-// [sys_off[s], sys_off[s+1]).  CTAs take systems from a queue ordered by
-// decreasing nnz (longest first) with one atomic fetch-add each; nothing
-// waits on another CTA.  Each CTA keeps its FP32 work vectors in its own
-// slot of a workspace sized for the largest system.
+// [sys_off[s], sys_off[s+1]).  Systems are taken from queues ordered by
+// decreasing nnz (longest first) with one atomic fetch-add each.
+//
+// Two kernels.  With one lane per row, a system of up to 65,536 rows of up to
+// 64 entries runs on a thread-block cluster of 1 to 7 CTAs, the smallest whose
+// shared memory holds its vectors (batched_cluster_kernel, over a sliced copy
+// of the matrices made when the batch is): one launch per cluster size, side by
+// side, the CTAs of a cluster meeting at cluster barriers.  All other systems,
+// and all of them with 2, 4 or 8 lanes per row, run on batched_cg_kernel: one
+// CTA per system at a time, its FP32 work vectors in the CTA's own slot of a
+// workspace sized for the largest system, no CTA waiting on another.
 //
 // Variants: G lanes per row (1 = one thread sums its row in order; 2/4/8 =
-// strided partial sums and a shuffle tree) x NT threads per CTA.  The
+// strided partial sums and a shuffle tree) x NT threads per CTA of
+// batched_cg_kernel; the clusters' CTAs have their own size.  The
 // autotuner (sk_batched_autotune) times every variant on a sample of the
-// batch and returns the fastest; the choice changes rounding only through
-// the row sums of G > 1.
+// batch and returns the fastest; the choice changes rounding through
+// the row sums of G > 1 and the order of the dot products' partial sums.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -1038,6 +1045,10 @@ SK_API sk_status sk_batched_autotune(sk_batch B, const double* b_dev, double* x_
   SK_CHECK(B && cfg && res && b_dev && x_dev && lanes_per_row && threads_per_cta, SK_INVALID_ARG,
            "null argument");
   const int limit = static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sample, B->nsys)));
+  // threads_per_cta is batched_cg_kernel's: with one lane per row and every
+  // sampled system on a cluster its variants are one launch, timed once
+  const bool clusters_only = B->cl_val && (B->cl_at.back().empty() || B->cl_at.back().front() >= limit);
+  float one_lane_ms = -1.0f;
   double best = 1e300;
   int best_i = 0;
   cudaEvent_t e0, e1;
@@ -1050,7 +1061,9 @@ SK_API sk_status sk_batched_autotune(sk_batch B, const double* b_dev, double* x_
     if (st != SK_OK) return st;
     BatchArgs a = make_args(B, ctas, b_dev, x_dev, cfg, res, limit);
     float ms = 0.0f;
-    for (int rep = 0; rep < 2; ++rep) {  // the first run warms the caches
+    const bool timed = v.G == 1 && clusters_only && one_lane_ms >= 0.0f;
+    if (timed) ms = one_lane_ms;
+    for (int rep = 0; rep < 2 && !timed; ++rep) {  // the first run warms the caches
       SK_CUDA(cudaMemsetAsync(x_dev, 0, B->nrow * sizeof(double), B->stream));
       SK_CUDA(cudaEventRecord(e0, B->stream));
       if ((st = enqueue_batch(B, v, ctas, a, limit)) != SK_OK) return st;
@@ -1058,6 +1071,7 @@ SK_API sk_status sk_batched_autotune(sk_batch B, const double* b_dev, double* x_
       SK_CUDA(cudaEventSynchronize(e1));
       SK_CUDA(cudaEventElapsedTime(&ms, e0, e1));
     }
+    if (v.G == 1) one_lane_ms = ms;
     if (ms_out) ms_out[i] = ms;
     if (ms < best) {
       best = ms;

@@ -997,8 +997,10 @@ class Batch_config:
 
 class Batch:
     """Many independent SPD systems (the diagonal blocks of one FP32 CSR
-    matrix) solved together on the device: one persistent launch, one CTA
-    per system, FP32 Jacobi-CG inside FP64 iterative refinement."""
+    matrix) solved together on the device: FP32 Jacobi-CG inside FP64
+    iterative refinement, a system on a thread-block cluster of 1 to 7 CTAs by
+    its size (lanes_per_row 1, at most 65,536 rows of at most 64 entries;
+    threads_per_cta does not apply to it) or on one CTA of threads_per_cta."""
 
     def __init__(self, sys_offsets, row_ptr, col_ind, values):
         sys_offsets = np.ascontiguousarray(sys_offsets, dtype=np.int64)
@@ -1029,7 +1031,9 @@ class Batch:
 
     def autotune(self, b, x, cfg=None, sample=512):
         """Times every (lanes_per_row, threads_per_cta) variant on the
-        `sample` largest systems; returns (lanes, threads, timings_ms)."""
+        `sample` largest systems; returns (lanes, threads, timings_ms).  The
+        one-lane variants are timed once where threads_per_cta applies to none
+        of those systems."""
         cfg = cfg or Batch_config()
         res, _ = self._results()
         g, t = ctypes.c_int32(), ctypes.c_int32()

@@ -1,5 +1,4 @@
-"""The batched solver (one persistent launch, FP32 Jacobi-CG inside FP64
-refinement per system) against the oracle's per-system FP64 Jacobi-CG: every
+"""The batched solver (FP32 Jacobi-CG inside FP64 refinement per system) against the oracle's per-system FP64 Jacobi-CG: every
 system reaches the FP64 tolerance on its true residual, with a comparable
 number of CG iterations."""
 import numpy as np
@@ -190,3 +189,17 @@ def test_results_go_to_the_arrays_of_the_call(gpu_lib, changed):
     for a, w in zip(new, want):
         assert torch.equal(a, w)
     assert (old[changed] == -7).all()
+
+
+def test_autotune_times_a_launch_once(gpu_lib):
+    """threads_per_cta does not apply to systems on clusters: the three one-lane
+    variants are one launch and one time, unless a sampled system stays with
+    the general kernel."""
+    import torch
+    for last, once in ((9000, True), (65600, False)):
+        offs, rp, ci, va, b = chains([300, 5000, last], seed=6)
+        B = gpu.Batch(offs, rp, ci, va)
+        bd = torch.from_numpy(b).cuda()
+        _, _, ms = B.autotune(bd, torch.zeros_like(bd), sample=3)
+        one_lane = ms.reshape(3, 4)[:, 0]
+        assert (ms > 0).all() and (np.unique(one_lane).size == 1) == once, ms
