@@ -815,7 +815,7 @@ sk_status enqueue_batch(sk_batch_s* B, const Variant& v, int ctas, BatchArgs a, 
 
 // Builds the sliced copy (from the CSR arrays on the device and the host row
 // pointers) of the systems that a class takes.  Without it (no such system,
-// too much padding, no memory) the batch runs on batched_cg_kernel.
+// too much padding) the batch runs on batched_cg_kernel.
 sk_status build_cluster_copy(sk_batch_s* B, const int64_t* sys_off, const int64_t* rp, const std::vector<int>& order) {
   for (int k = 0; k < kNumClasses; ++k) B->cl_ctas[k] = cluster_ctas(kClasses[k]);
   std::vector<int> cls(static_cast<size_t>(B->nsys), kNumClasses), slice0(static_cast<size_t>(B->nsys) + 1), off;
@@ -861,33 +861,49 @@ sk_status build_cluster_copy(sk_batch_s* B, const int64_t* sys_off, const int64_
     B->cl_first.push_back(static_cast<int>(flat.size()));
     flat.insert(flat.end(), l.begin(), l.end());
   }
-  auto alloc = [&](size_t bytes, const void* src) -> void* {
-    void* m = nullptr;
-    if (cudaMalloc(&m, bytes + 64) != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    B->allocs.push_back(m);
-    if (src && cudaMemcpy(m, src, bytes, cudaMemcpyHostToDevice) != cudaSuccess) return nullptr;
-    return m;
+  void *d_slice0 = nullptr, *d_off = nullptr, *d_order = nullptr, *d_len = nullptr, *d_col = nullptr, *d_val = nullptr;
+  auto alloc = [&](void** m, size_t bytes, const void* src) -> sk_status {
+    SK_CUDA(cudaMalloc(m, bytes + 64));
+    B->allocs.push_back(*m);
+    if (src) SK_CUDA(cudaMemcpy(*m, src, bytes, cudaMemcpyHostToDevice));
+    return SK_OK;
   };
-  B->cl_slice0 = static_cast<int*>(alloc(slice0.size() * 4, slice0.data()));
-  B->cl_off = static_cast<int*>(alloc(off.size() * 4, off.data()));
-  B->cl_order = static_cast<int*>(alloc(flat.size() * 4, flat.data()));
-  B->cl_len = static_cast<unsigned char*>(alloc(static_cast<size_t>(slices) * 32, nullptr));
-  B->cl_col = static_cast<unsigned short*>(alloc(static_cast<size_t>(entries) * 2, nullptr));
-  float* val = static_cast<float*>(alloc(static_cast<size_t>(entries) * 4, nullptr));
-  if (!B->cl_slice0 || !B->cl_off || !B->cl_order || !B->cl_len || !B->cl_col || !val) return SK_OK;
+  sk_status s;
+  if ((s = alloc(&d_slice0, slice0.size() * 4, slice0.data())) != SK_OK ||
+      (s = alloc(&d_off, off.size() * 4, off.data())) != SK_OK ||
+      (s = alloc(&d_order, flat.size() * 4, flat.data())) != SK_OK ||
+      (s = alloc(&d_len, static_cast<size_t>(slices) * 32, nullptr)) != SK_OK ||
+      (s = alloc(&d_col, static_cast<size_t>(entries) * 2, nullptr)) != SK_OK ||
+      (s = alloc(&d_val, static_cast<size_t>(entries) * 4, nullptr)) != SK_OK)
+    return s;
   for (int k = 0; k <= kNumClasses; ++k) {
     SK_CUDA(cudaStreamCreateWithFlags(&B->fork[k], cudaStreamNonBlocking));
     SK_CUDA(cudaEventCreateWithFlags(&B->ev_join[k], cudaEventDisableTiming));
   }
   SK_CUDA(cudaEventCreateWithFlags(&B->ev_fork, cudaEventDisableTiming));
-  cl_fill_kernel<<<static_cast<unsigned>(B->nsys), 256, 0, B->stream>>>(view_of(B), B->cl_slice0, B->cl_off,
-                                                                        B->cl_len, B->cl_col, val);
+  cl_fill_kernel<<<static_cast<unsigned>(B->nsys), 256, 0, B->stream>>>(
+      view_of(B), static_cast<int*>(d_slice0), static_cast<int*>(d_off), static_cast<unsigned char*>(d_len),
+      static_cast<unsigned short*>(d_col), static_cast<float*>(d_val));
   SK_CUDA(cudaGetLastError());
   SK_CUDA(cudaStreamSynchronize(B->stream));
-  B->cl_val = val;
+  B->cl_slice0 = static_cast<int*>(d_slice0);
+  B->cl_off = static_cast<int*>(d_off);
+  B->cl_order = static_cast<int*>(d_order);
+  B->cl_len = static_cast<unsigned char*>(d_len);
+  B->cl_col = static_cast<unsigned short*>(d_col);
+  B->cl_val = static_cast<float*>(d_val);
+  return SK_OK;
+}
+
+// The copy if the device has room for it; else what it took is given back and
+// the batch runs on batched_cg_kernel.
+sk_status try_cluster_copy(sk_batch_s* B, const int64_t* sys_off, const int64_t* rp, const std::vector<int>& order) {
+  const size_t mark = B->allocs.size();
+  const sk_status s = build_cluster_copy(B, sys_off, rp, order);
+  if (s != SK_OUT_OF_MEMORY) return s;
+  cudaGetLastError();
+  for (size_t k = mark; k < B->allocs.size(); ++k) cudaFree(B->allocs[k]);
+  B->allocs.resize(mark);
   return SK_OK;
 }
 
@@ -967,7 +983,7 @@ SK_API sk_status sk_batch_create(sk_batch* out, int64_t nsys, const int64_t* sys
   B->counter = static_cast<int*>(c);
   if (nnz) cudaMemcpy(v, values, nnz * 4, cudaMemcpyHostToDevice);
   std::vector<int> queue(order.begin(), order.end());
-  if ((st = build_cluster_copy(B, sys_offsets, row_ptr, queue)) != SK_OK) {
+  if ((st = try_cluster_copy(B, sys_offsets, row_ptr, queue)) != SK_OK) {
     sk_batch_destroy(B);
     return st;
   }

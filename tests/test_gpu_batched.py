@@ -203,3 +203,28 @@ def test_autotune_times_a_launch_once(gpu_lib):
         _, _, ms = B.autotune(bd, torch.zeros_like(bd), sample=3)
         one_lane = ms.reshape(3, 4)[:, 0]
         assert (ms > 0).all() and (np.unique(one_lane).size == 1) == once, ms
+
+
+def test_no_room_for_the_sliced_copy(gpu_lib):
+    """A device with room for the matrices and half of their sliced copy: the
+    batch gives that half back and its systems are solved without it."""
+    import gc
+
+    import torch
+    small = chains([100], seed=1)
+    gpu.Batch(*small[:4]).solve(torch.from_numpy(small[4]).cuda(), torch.zeros(100, dtype=torch.float64, device="cuda"))
+    offs, rp, ci, va, b = chains([60000] * 128, seed=7)
+    csr, copy = 8 * ci.size + 4 * rp.size, 6 * ci.size
+    gc.collect()  # no batch of another test is given back in between
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    held = torch.empty(free - csr - copy // 2 - (8 << 20), dtype=torch.uint8, device="cuda")
+    before = torch.cuda.mem_get_info()[0]
+    B = gpu.Batch(offs, rp, ci, va)
+    taken = before - torch.cuda.mem_get_info()[0]
+    del held
+    torch.cuda.empty_cache()
+    assert taken <= csr + (16 << 20), (taken, csr, copy)
+    bd = torch.from_numpy(b).cuda()
+    _, _, rel, conv = B.solve(bd, torch.zeros_like(bd))
+    assert conv.all() and (rel < 1e-10).all()
