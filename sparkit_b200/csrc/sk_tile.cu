@@ -11,9 +11,9 @@
 // from shared memory.  The entries a row has in one panel are a segment; the
 // segments of a panel are sorted by decreasing length and packed 32 to a
 // slice, a lane each, entry j of lane l at off + 32 j + l with a 16-bit column
-// inside the panel.  A lane sums its segment from first to last entry; the row's
-// partial sums are stored together in panel order and added by the kernel that
-// takes the short rows.
+// inside the panel.  A lane sums its segment, eight entries at a time as a
+// tree; the row's partial sums are stored together in panel order and added by
+// the kernel that takes the short rows.
 //
 // Built on the device: a search per (row, panel), a radix sort of the
 // segments by (panel, decreasing length), a scan of the slices' sizes and one
@@ -140,8 +140,8 @@ sk_status build_tiles(sk_matrix A, i64 long_nnz, i64 longest, cudaStream_t st) {
     return SK_OK;
   const size_t V = vbytes(A->dtype);
   // as many panels as shared memory asks for, and so many that a row's
-  // segments stay short when its columns are spread: a lane sums a segment
-  // entry after entry (one panel of 2048-entry rows took 120 us however few)
+  // segments stay short when its columns are spread: a segment is one lane's
+  // chain (one panel of 2048-entry rows took 120 us however few)
   const i64 least = std::max((A->ncol * static_cast<i64>(V) + kTileSmem - 1) / kTileSmem,
                              (longest + kTileSegment - 1) / kTileSegment);
   const int width = static_cast<int>(((A->ncol + least - 1) / least + 31) / 32 * 32);

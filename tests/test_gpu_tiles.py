@@ -87,6 +87,37 @@ def test_streams_and_capture(gpu_lib, oracle):
     held(A, xs[0].cpu().numpy(), y.cpu().numpy(), oracle)
 
 
+@pytest.mark.parametrize("dtype,n", [(np.float64, 150_000), (np.float32, 300_000)])
+@pytest.mark.parametrize("spread", [1, 3])
+def test_long_rows_round_no_worse_than_split(gpu_lib, dtype, n, spread):
+    """The long rows' error against wider arithmetic (80 bits for FP64, 64 for
+    FP32) beside that of the split product, which a captured call runs: rows
+    spread over all panels, and rows crowded into a third of them.  A lane
+    adds eight trees of eight entries one after another and up to six such runs,
+    the split product 16 entries of a row of 2048; rows of a few hundred
+    crowded entries may come 10% higher, which the bar leaves them."""
+    import torch
+    m = 1_000_003
+    A = skewed(n, m // spread, 8, dtype)
+    A = formats.Compressed_row_matrix((n, m), A.row_ptr(), A.col_ind(), A.values())
+    Ad = gpu.Device_matrix(A)
+    x = matgen.uniform_vector(m, seed=9, dtype=dtype)
+    xd = torch.from_numpy(x).cuda()
+    direct, split = torch.empty(n, dtype=xd.dtype, device="cuda"), torch.empty(n, dtype=xd.dtype, device="cuda")
+    assert launches(lambda: Ad.spmv(xd, direct)) == 2
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        Ad.spmv(xd, split)
+    g.replay()
+    torch.cuda.synchronize()
+    wide = np.longdouble if dtype == np.float64 else np.float64
+    long = A.row_lengths() > 32
+    terms = A.values().astype(wide) * x[A.col_ind()].astype(wide)
+    exact = np.add.reduceat(terms, A.row_ptr()[:-1])  # every row holds at least one entry
+    err = [np.linalg.norm((y.cpu().numpy().astype(wide) - exact)[long].astype(np.float64)) for y in (direct, split)]
+    assert err[0] <= 1.1 * err[1], err
+
+
 def test_where_the_copy_is_not_built(gpu_lib, oracle):
     """Few long-row entries, or a long row whose columns do not ascend: one
     launch, as before."""
