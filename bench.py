@@ -251,14 +251,10 @@ def time_device(fn, steps, warmup, stream):
     return e0.elapsed_time(e1) / steps  # ms per step
 
 
-def layout_bytes(Ad, dtype):
-    """Bytes of one product on the layout the handle runs on: of the stencil
-    copy of a symmetric 7-point matrix 4 planes, the row masks, x and y; else
-    the handle's own byte model."""
-    info = Ad.info()
-    if Ad.layout() == "stencil":
-        return info["nrow"] * (6 * np.dtype(dtype).itemsize + 2)
-    return info["spmv_bytes"]
+def format_bytes(A, vbytes=8):
+    """The byte model of a product in the CSR format: the matrix, x and y once."""
+    n, m = A.shape()
+    return (vbytes + 4) * A.size() + 4 * (n + 1) + vbytes * (n + m)
 
 
 def rotate(make, bytes_one, total=300e6):
@@ -287,24 +283,17 @@ def sweep(stream, grid):
         Adt = A.astype(dt)
         xd = torch.from_numpy(x.astype(dt)).cuda()
         yd = torch.empty_like(xd)
-        # the FP32 diagonal copy with x and y (80 MB at 128^3) would sit in
-        # the L2 between products, so the copy is timed in FP64 only (155 MB)
-        for fmt, M in (("csr", Adt), ("ell", formats.to_ellpack(Adt)), ("jad", formats.to_jagged_diagonal(Adt)),
-                       ("csr_diagonal_copy", Adt if tag == "f64" else None)):
-            if M is None:
-                continue
+        for fmt, M in (("csr", Adt), ("ell", formats.to_ellpack(Adt)), ("jad", formats.to_jagged_diagonal(Adt))):
             Ad = gpu.Device_matrix(M)
-            if fmt == "csr_diagonal_copy":
-                assert Ad.add_diagonals()
-            step, copies = rotate(lambda: (gpu.Device_matrix(M), xd.clone(), yd.clone(), sptr), layout_bytes(Ad, dt))
-            ms = time_device(step, 300, 20, stream)
-            # spmv_bytes is the byte model of the format (for the diagonal
-            # copy: its values and row masks, x and y), layout_bytes that of
-            # the copy the product runs on
             info = Ad.info()
-            out[f"lap3d_{fmt}_{tag}"] = {"gbs": info["spmv_bytes"] / ms / 1e6, "us": ms * 1e3,
-                                         "bytes": info["spmv_bytes"], "layout": Ad.layout(),
-                                         "layout_bytes": layout_bytes(Ad, dt),
+            step, copies = rotate(lambda: (gpu.Device_matrix(M), xd.clone(), yd.clone(), sptr), info["spmv_bytes"])
+            ms = time_device(step, 300, 20, stream)
+            # the byte model of the format; spmv_bytes is that of the copy a
+            # CSR product runs on
+            bytes_fmt = format_bytes(Adt, np.dtype(dt).itemsize) if fmt == "csr" else info["spmv_bytes"]
+            out[f"lap3d_{fmt}_{tag}"] = {"gbs": bytes_fmt / ms / 1e6, "us": ms * 1e3,
+                                         "bytes": bytes_fmt, "layout": Ad.layout(),
+                                         "layout_bytes": info["spmv_bytes"],
                                          "device_bytes": info["device_bytes"]}
             for c in copies:
                 c[0].close()
@@ -705,41 +694,8 @@ def solver_runs(grid3):
         if name == "mixed_fp32_fp64":
             res["speedup_mixed_vs_plain"] = tp / tm
     res["reps_ms"] = {"plain_fp64": reps_p, "mixed": reps_m, "reported": "best of the repetitions after the first"}
-    # the same two solvers on a handle carrying the diagonal copy (one value
-    # plane per stencil offset, no column indices, x read contiguously);
-    # every product keeps its bits, so the iteration counts are the CSR ones
     JG.close()
     Gd.close()
-    Dd = gpu.Device_matrix(G)
-    dia = {"built": Dd.add_diagonals()}
-    Dd.add_f32_values()
-    JD = gpu.jacobi(Dd)
-    for name, solve in (("plain_fp64", lambda x: gpu.conjugate_gradient(
-                            bd, x, gpu.CGConfig(1e-10, 10 ** 6, 200000), gpu.spmv(Dd), JD)),
-                        ("mixed_fp32_fp64", lambda x: gpu.mixed_cg(
-                            bd, x, gpu.Mixed_config(1e-10, 1e-5, 100, 200000), gpu.spmv(Dd)))):
-        reps = []
-        for rep in range(3):
-            xd = torch.zeros_like(bd)
-            torch.cuda.synchronize()
-            t0 = time.perf_counter()
-            sv = solve(xd)
-            torch.cuda.synchronize()
-            reps.append((time.perf_counter() - t0) * 1e3)
-        rel = float(np.linalg.norm(b - gpu.multiply(Dd, xd.cpu().numpy())) / np.linalg.norm(b))
-        entry = {"ms": min(reps[1:]), "reps_ms": reps, "converged": sv.converged, "true_rel_residual": rel}
-        if name == "plain_fp64":
-            entry["iterations"] = sv.computed_iterations
-        else:
-            entry.update({"outer": sv.outer_iterations, "inner_iterations": sv.inner_iterations,
-                          "persistent": sv.persistent, "inner_ms": sv.inner_ms,
-                          "us_per_inner_iteration": sv.inner_ms * 1e3 / max(sv.inner_iterations, 1)})
-        dia[name] = entry
-    dia["speedup_mixed_vs_plain"] = dia["plain_fp64"]["ms"] / dia["mixed_fp32_fp64"]["ms"]
-    dia["speedup_mixed_vs_plain_csr"] = res["plain_fp64"]["ms"] / dia["mixed_fp32_fp64"]["ms"]
-    res["diagonal_copy"] = dia
-    JD.close()
-    Dd.close()
     res["n"] = n
     res["nnz"] = G.size()
     out[f"c3_grf_diffusion_{grid3}cubed"] = res
@@ -995,12 +951,6 @@ def profile_formats(grid):
             Ad.spmv(xd, yd)
             torch.cuda.synchronize()
             Ad.close()
-        if dt == np.float64:  # the CSR handle through its diagonal copy
-            Ad = gpu.Device_matrix(Adt)
-            assert Ad.add_diagonals()
-            Ad.spmv(xd, yd)
-            torch.cuda.synchronize()
-            Ad.close()
     B = matgen.vector_laplacian_3d_bsr(grid // 2, seed=1)
     Bd = gpu.Device_matrix(B)
     xb = torch.from_numpy(matgen.uniform_vector(B.shape()[0], seed=2)).cuda()
@@ -1230,10 +1180,9 @@ def main():
     A, x = build_workload(args.grid)
     n = A.shape()[0]
     Ad = gpu.Device_matrix(A)
-    info = Ad.info()
-    bytes_one = info["spmv_bytes"]
+    bytes_one = format_bytes(A)
     xd = torch.from_numpy(x).cuda()
-    moved = layout_bytes(Ad, np.float64)
+    moved = Ad.info()["spmv_bytes"]
     step, copies = rotate(lambda: (gpu.Device_matrix(A), xd.clone(), torch.empty_like(xd), sptr), moved)
 
     try:

@@ -203,7 +203,8 @@ SK_API sk_status sk_matrix_destroy(sk_matrix A);
 
 /* info[0..7] = format, dtype, nrow, ncol, nnz (stored entries), width
  * (ELL width / JAD diagonal count / BSR block count), device bytes held,
- * algorithmic bytes of one FP SpMV (the roofline byte model). */
+ * algorithmic bytes of one FP SpMV (the roofline byte model): the format's,
+ * or the copy's where the product runs on a stencil or diagonal copy. */
 SK_API sk_status sk_matrix_info(sk_matrix A, int64_t info[8]);
 
 /* The device layout the product of a handle runs on (chosen at upload; the
@@ -211,7 +212,8 @@ SK_API sk_status sk_matrix_info(sk_matrix A, int64_t info[8]);
  *   SK_LAYOUT_NATIVE    the handle's own format (CSR: row tiles);
  *   SK_LAYOUT_SELL      SELL-32 copy (CSR rows of at most 64 entries; 2x2
  *                       and 3x3 BSR);
- *   SK_LAYOUT_DIAGONALS diagonal copy (sk_matrix_add_diagonals);
+ *   SK_LAYOUT_DIAGONALS diagonal copy (sk_matrix_add_diagonals, on a handle
+ *                       without a stencil copy);
  *   SK_LAYOUT_SPLIT     CSR split by row length (skewed rows);
  *   SK_LAYOUT_PANELS    CSR column panels (sk_matrix_add_panels: x staged
  *                       panel by panel in shared memory, every row summed
@@ -234,7 +236,12 @@ SK_API sk_status sk_matrix_add_f32_values(sk_matrix A);
  * on the handle (sk_spmv, sk_spmv_host, the solvers' steps, the per-step
  * FP32 inner solve of the mixed solver) read it instead of the CSR arrays:
  * no column indices and no gathered x, and each row summed over its stored
- * entries in its CSR order, so the results keep their bits.  The persistent
+ * entries in its CSR order, so the results keep their bits.  A handle with a
+ * stencil copy (SK_LAYOUT_STENCIL) needs it less: sk_spmv and the solvers'
+ * steps in the handle's own type stay on the stencil copy, which holds the
+ * same diagonals or half of them (FP64, 128^3 Laplacian: 19.3 us a product, 26.2
+ * over the diagonal copy), and the diagonal copy serves sk_spmv_host and the
+ * FP32 products of an FP64 handle.  The persistent
  * FP32 inner solve of the mixed solver reads it too, at two CTAs per SM
  * (its dot products then sum in another order than over SELL-32).
  * No reference counterpart: a device layout of Compressed_row_matrix

@@ -447,7 +447,9 @@ i64 sk_matrix_s::spmv_bytes() const {
   const i64 V = dtype == SK_F64 ? 8 : 4;
   switch (format) {
     case SK_CSR:
-      if (csr.dia_n) return (V * csr.dia_n + 2) * nrow + V * ncol + V * nrow;  // planes, mask, x, y
+      // planes, mask, x, y; the stencil copy is read before the diagonal one
+      if (csr.st_n) return (V * (csr.st_sym ? csr.st_n - csr.st_n / 2 : csr.st_n) + 2) * nrow + V * ncol + V * nrow;
+      if (csr.dia_n) return (V * csr.dia_n + 2) * nrow + V * ncol + V * nrow;
       return V * nnz + 4 * nnz + 4 * (nrow + 1) + V * ncol + V * nrow;
     case SK_ELL: return (V + 4) * nnz + V * ncol + V * nrow;
     case SK_JAD: return (V + 4) * nnz + 4 * (jad.njd + 1) + 4 * nrow + V * ncol + V * nrow;

@@ -229,7 +229,9 @@ class Device_matrix:
 
     def add_diagonals(self):
         """Adds the diagonal copy of a stencil-pattern CSR handle; False when
-        the pattern does not qualify (the handle is then unchanged)."""
+        the pattern does not qualify (the handle is then unchanged).  Where
+        layout() is "stencil", products in the handle's own type stay on that
+        copy."""
         built = ctypes.c_int(0)
         check(lib().sk_matrix_add_diagonals(self.handle, ctypes.byref(built)))
         return bool(built.value)

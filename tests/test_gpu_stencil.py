@@ -70,3 +70,29 @@ def test_solver_over_the_copy(gpu_lib, oracle):
     assert s.converged and abs(s.computed_iterations - sr["computed_iterations"]) <= max(
         2, sr["computed_iterations"] // 50)
     assert np.linalg.norm(b - oracle.spmv(A, x)) <= 1e-9 * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_diagonal_copy_beside_it(gpu_lib, oracle, symmetric):
+    """sk_matrix_add_diagonals on a handle with a stencil copy: its products
+    stay on that copy, whose bytes the handle reports before and after, and
+    every entry point keeps its bits."""
+    import torch
+    A = grid((43, 47, 53), symmetric, 4)
+    n = A.shape()[0]
+    Ad = gpu.Device_matrix(A)
+    moved = n * (8 * (4 if symmetric else 7) + 2 + 16)
+    assert Ad.info()["spmv_bytes"] == moved
+    x = matgen.uniform_vector(n, seed=6)
+    want = oracle.spmv(A, x)
+    assert Ad.add_diagonals()
+    assert Ad.layout() == "stencil" and Ad.info()["spmv_bytes"] == moved
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty_like(xd)
+    Ad.spmv(xd, yd)
+    assert np.array_equal(yd.cpu().numpy(), want)
+    assert np.array_equal(gpu.multiply(Ad, x), want)
+    Ad.add_f32_values()
+    y32 = torch.empty(n, dtype=torch.float32, device="cuda")
+    Ad.spmv_f32(xd.float(), y32)
+    assert np.array_equal(y32.cpu().numpy(), oracle.spmv(A.astype(np.float32), x.astype(np.float32)))
