@@ -202,6 +202,13 @@ sk_status csr_symmetric(sk_matrix A, std::vector<int> const& offs, bool* sym) {
   return SK_OK;
 }
 
+// Whether a place in nd planes of n rows, the padding of the last 32-row slice
+// with it, is an int: stencil_spmv_kernel reads absent entries there too.
+static constexpr bool planes_fit_int(i64 n, i64 nd) { return (n + 31) / 32 * 32 * nd < (i64(1) << 31) - 64; }
+// the last slice alone reaches past it: n * nd < 2^31 - 64 does not say enough
+static_assert(!planes_fit_int(306783361, 7) && 306783361ll * 7 < (1ll << 31) - 64 && planes_fit_int(306783328, 7));
+static_assert(!planes_fit_int(429496705, 5) && 429496705ll * 5 < (1ll << 31) - 64 && planes_fit_int(429496672, 5));
+
 sk_status build_stencil(sk_matrix A) {
   const i64 n = A->nrow;
   if (A->format != SK_CSR || n != A->ncol || A->nnz < kStencilMinEntries) return SK_OK;
@@ -209,7 +216,7 @@ sk_status build_stencil(sk_matrix A) {
   sk_status s = dia_pattern(A, &offs);
   if (s != SK_OK) return s;
   const int nd = static_cast<int>(offs.size());
-  if ((nd != 5 && nd != 7) || n * nd >= (i64(1) << 31) - 64) return SK_OK;
+  if ((nd != 5 && nd != 7) || !planes_fit_int(n, nd)) return SK_OK;
   bool sym = false;
   if ((s = csr_symmetric(A, offs, &sym)) != SK_OK) return s;
   const int first = sym ? nd / 2 : 0;
