@@ -214,7 +214,16 @@ SK_API sk_status sk_matrix_info(sk_matrix A, int64_t info[8]);
  *                       and 3x3 BSR);
  *   SK_LAYOUT_DIAGONALS diagonal copy (sk_matrix_add_diagonals, on a handle
  *                       without a stencil copy);
- *   SK_LAYOUT_SPLIT     CSR split by row length (skewed rows);
+ *   SK_LAYOUT_SPLIT     CSR split by row length (skewed rows): rows of up to 32
+ *                       entries summed in storage order, longer ones in a
+ *                       fixed tree.  With at least 8M entries (FP64; FP32: 16M)
+ *                       in the longer rows there are two trees, of like
+ *                       rounding error: one over panels of x, and, for a
+ *                       product that is being captured (the solvers' graphs of
+ *                       steps among them), the one of smaller handles, since a
+ *                       replay cannot take its turn at the handle's partial
+ *                       sums.  Either gives the same bits on every call;
+ *                       between them the last bits of longer rows differ;
  *   SK_LAYOUT_PANELS    CSR column panels (sk_matrix_add_panels: x staged
  *                       panel by panel in shared memory, every row summed
  *                       in column order);
@@ -260,9 +269,9 @@ SK_API sk_status sk_matrix_add_diagonals(sk_matrix A, int* built);
  * each CTA walks column panels of x staged in shared memory with a running
  * sum per row of its block, and the matrix stream arrives by bulk copies.
  * It costs 10 (FP64) or 6 (FP32) bytes per entry beside the CSR arrays.
- * On the Zipf-row matrix of the sweep it runs at 0.79x the speed of the
+ * On the Zipf-row matrix of the sweep it runs at 0.45x the speed of the
  * default split product, which sums rows longer than 32 entries in a
- * fixed tree.  *built is 1 when the handle has the copy, 0 when it does
+ * fixed tree, and at 0.86x of that product's captured form.  *built is 1 when the handle has the copy, 0 when it does
  * not qualify (SELL-32 or diagonal copy present, a row whose columns do
  * not ascend, or rows too many for a block's running sums); the handle is
  * unchanged then. */

@@ -414,9 +414,10 @@ sell_spmv_kernel(int nrow, const int* __restrict__ off, const unsigned char* __r
 // row order, one thread per row, each summed in storage order from 0 (the
 // bits of sparse_blas.hpp:25-28).  No shared memory, so the L1 serves the
 // random gathers of x only.
+//
+// TILE: tile_part_kernel has summed the long rows' entries, and a long row is
+// the sum of its partial sums, eight lanes to a row.
 // ------------------------------------------------------------------
-// With TILE the long rows' entries were summed by tile_part_kernel and a long
-// row is the sum of its partial sums, taken the same way.
 template <typename T, class Epi, int MINB, bool TILE>
 __global__ void __launch_bounds__(kThreads, MINB)
 hyb_spmv_kernel(const int* __restrict__ rp, const int* __restrict__ ci, const T* __restrict__ va,
@@ -453,26 +454,27 @@ hyb_spmv_kernel(const int* __restrict__ rp, const int* __restrict__ ci, const T*
         for (int o = 4; o > 0; o >>= 1) sum = add(sum, __shfl_xor_sync(grp, sum, o));
         if (l8 == 0) reduce_terms<NR>(ws, row, red, [&](double* rr) { epi(row, sum, rr); });
       }
-    } else
-    for (int w = (static_cast<int>(blockIdx.x) - short_ctas) * W + (threadIdx.x >> 5); w < nlong; w += nw) {
-      const int row = __ldg(long_rows + w);
-      const int b = __ldg(rp + row), e = __ldg(rp + row + 1);
-      T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
-      int k = b + lane;
-      for (; k + 96 < e; k += 128) {
-        const int c0 = __ldcs(ci + k), c1 = __ldcs(ci + k + 32), c2 = __ldcs(ci + k + 64), c3 = __ldcs(ci + k + 96);
-        const T v0 = __ldcs(va + k), v1 = __ldcs(va + k + 32), v2 = __ldcs(va + k + 64), v3 = __ldcs(va + k + 96);
-        const T x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
-        a0 = add(a0, mul(v0, x0));
-        a1 = add(a1, mul(v1, x1));
-        a2 = add(a2, mul(v2, x2));
-        a3 = add(a3, mul(v3, x3));
-      }
-      for (; k < e; k += 32) a0 = add(a0, mul(__ldcs(va + k), __ldg(x + __ldcs(ci + k))));
-      T sum = add(add(a0, a1), add(a2, a3));
+    } else {
+      for (int w = (static_cast<int>(blockIdx.x) - short_ctas) * W + (threadIdx.x >> 5); w < nlong; w += nw) {
+        const int row = __ldg(long_rows + w);
+        const int b = __ldg(rp + row), e = __ldg(rp + row + 1);
+        T a0 = T(0), a1 = T(0), a2 = T(0), a3 = T(0);
+        int k = b + lane;
+        for (; k + 96 < e; k += 128) {
+          const int c0 = __ldcs(ci + k), c1 = __ldcs(ci + k + 32), c2 = __ldcs(ci + k + 64), c3 = __ldcs(ci + k + 96);
+          const T v0 = __ldcs(va + k), v1 = __ldcs(va + k + 32), v2 = __ldcs(va + k + 64), v3 = __ldcs(va + k + 96);
+          const T x0 = __ldg(x + c0), x1 = __ldg(x + c1), x2 = __ldg(x + c2), x3 = __ldg(x + c3);
+          a0 = add(a0, mul(v0, x0));
+          a1 = add(a1, mul(v1, x1));
+          a2 = add(a2, mul(v2, x2));
+          a3 = add(a3, mul(v3, x3));
+        }
+        for (; k < e; k += 32) a0 = add(a0, mul(__ldcs(va + k), __ldg(x + __ldcs(ci + k))));
+        T sum = add(add(a0, a1), add(a2, a3));
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum = add(sum, __shfl_xor_sync(0xffffffffu, sum, o));
-      if (lane == 0) reduce_terms<NR>(ws, row, red, [&](double* rr) { epi(row, sum, rr); });
+        for (int o = 16; o > 0; o >>= 1) sum = add(sum, __shfl_xor_sync(0xffffffffu, sum, o));
+        if (lane == 0) reduce_terms<NR>(ws, row, red, [&](double* rr) { epi(row, sum, rr); });
+      }
     }
   } else {
     for (int t = blockIdx.x * kThreads + threadIdx.x; t < nshort; t += short_ctas * kThreads) {
