@@ -63,7 +63,9 @@ def test_cpp_dropin_misuse_does_not_compile(case, message):
 @pytest.mark.gpu
 def test_cpp_dropin_on_gpu():
     exe = os.path.join(BUILD, "dropin_test")
-    assert os.path.isfile(exe), "tests/cpp/_build/dropin_test is built by tests/cpp/build.sh where the reference is"
+    if not os.path.isfile(os.path.join(ROOT, "oracle", "_ref", "libsparkit_ref.so")):
+        pytest.skip("the C++ drop-in test is built where the reference is: neither it nor the compiled reference is here")
+    assert os.path.isfile(exe), "tests/cpp/build.sh builds tests/cpp/_build/dropin_test beside the compiled reference"
     out = subprocess.run([exe, "gpu"], capture_output=True, text=True, timeout=600)
     print(out.stdout)
     assert out.returncode == 0, out.stdout + out.stderr
