@@ -205,3 +205,32 @@ def test_coarse_corrected_smoother_gain_at_128(gpu_lib, oracle, torch):
     assert res["learned"][2] < 1.5e-8, res
     assert 2 * res["learned"][1] <= res["jacobi"][1], res
     assert res["learned"][3] < res["jacobi"][3], res
+
+
+@pytest.mark.parametrize("nx", [1184, 1216, 2368, 2432, 4736, 4800])
+def test_forward_where_layers_split_over_channels(gpu_lib, oracle, torch, nx):
+    """A layer of t tiles of 8 x 16 cells gives each tile a CTA per 16 output
+    channels while that makes 148 CTAs at most, a 64-channel one a CTA per 32
+    channels next.  On a grid of 32 rows level l has nx / 2^l / 8 tiles: 74 and
+    76 on levels 1, 2 and 3 (37 and 38 on the next) with these sizes."""
+    test_planes_and_forward_match_oracle(gpu_lib, oracle, torch, nx, 32)
+
+
+def test_gradients_one_after_another(gpu_lib, oracle, torch):
+    """Calls with other batch sizes, back to back on one net (their weight
+    gradients run on a stream beside the chain): each gives the bits of a
+    net of its own."""
+    nx, ny = 64, 48
+    A = rect_convdiff(nx, ny, 5)
+    pairs = gpu.Pairs(nx, ny, 8, 1)
+    inst = pairs.add_instance(gpu.Device_matrix(A))
+    rng = np.random.default_rng(6)
+    for _ in range(8):
+        e = rng.standard_normal(nx * ny)
+        pairs.add(inst, torch.from_numpy(oracle.spmv(A, e)).cuda(), torch.from_numpy(e).cuda())
+    batches = [list(range(8)), [5], [1, 7, 2], list(range(7, -1, -1)), [5]]
+    net = gpu.Net(seed=9)
+    got = [net.loss_grad(pairs, idx, 0.5) for idx in batches]
+    for idx, (loss, grad) in zip(batches, got):
+        want_loss, want = gpu.Net(seed=9).loss_grad(pairs, idx, 0.5)
+        assert loss == want_loss and np.array_equal(grad, want) and np.isfinite(grad).all()

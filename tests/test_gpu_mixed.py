@@ -198,3 +198,39 @@ def test_mixed_fgmres_refuses_the_network(gpu_lib):
     with pytest.raises(_lib.SkError) as e:
         gpu.mixed_fgmres(bd, torch.zeros_like(bd), gpu.Mixed_fgmres_config(), gpu.spmv(Ad), L)
     assert e.value.status == 9
+
+
+def _scaled_laplacian_2d(m):
+    """D L D with positive D: a variable 5-point SPD matrix, symmetric bit for bit."""
+    from sparkit_b200.formats import Compressed_row_matrix
+    L = matgen.laplacian_2d_dirichlet(m, m + 3)
+    n = L.shape()[0]
+    d = np.exp(np.random.default_rng(m).uniform(-0.5, 0.5, n))
+    rows = np.repeat(np.arange(n), np.diff(L.row_ptr()))
+    return Compressed_row_matrix((n, n), L.row_ptr(), L.col_ind(), L.values() * (d[rows] * d[L.col_ind()]))
+
+
+@pytest.mark.parametrize("points", [5, 7])
+def test_inner_planes_of_a_matrix_one_bit_off_symmetric(gpu_lib, oracle, points):
+    """The scaled planes of a 5- or 7-point matrix are stored once when it is
+    symmetric bit for bit and in full when one entry differs in its last bit:
+    both reach the tolerance, in the same number of inner steps to 2% (the
+    matrices differ by 1e-16, the planes' entries by their rounding)."""
+    import torch
+    from sparkit_b200.formats import Compressed_row_matrix
+    A = _scaled_laplacian_2d(61) if points == 5 else matgen.diffusion_3d_grf(23, sigma=1.0, corr_len=4.0, seed=5)
+    n = A.shape()[0]
+    at = A.row_ptr()[n // 2]  # the first entry of a middle row: below the diagonal
+    assert A.col_ind()[at] < n // 2
+    v = A.values().copy()
+    v[at] = np.nextafter(v[at], 0.0)
+    b = matgen.uniform_vector(n, seed=8)
+    bd = torch.from_numpy(b).cuda()
+    inner = []
+    for M in (A, Compressed_row_matrix((n, n), A.row_ptr(), A.col_ind(), v)):
+        xd = torch.zeros_like(bd)
+        s = gpu.mixed_cg(bd, xd, gpu.Mixed_config(1e-10, 1e-5, 50, 100000), gpu.spmv(gpu.Device_matrix(M)))
+        rel = np.linalg.norm(b - oracle.spmv(M, xd.cpu().numpy())) / np.linalg.norm(b)
+        assert s.converged and s.persistent and rel < 1e-10, (s, rel)
+        inner.append(s.inner_iterations)
+    assert abs(inner[0] - inner[1]) <= max(2, 0.02 * inner[0]), inner

@@ -416,3 +416,44 @@ def test_small_minres_runs_as_one_launch(gpu_lib, oracle, sides):
     assert len(s.iteration_residuals) == s.computed_iterations
     np.testing.assert_allclose(s.iteration_residuals[0], sr["iteration_residuals"][0], rtol=1e-10)
     assert np.linalg.norm(b - oracle.spmv(A, x)) <= 1e-9 * np.linalg.norm(b)
+
+
+def _banded(n, offsets):
+    """SPD, diagonally dominant, -1 on the given diagonals and their mirrors."""
+    from sparkit_b200.formats import Compressed_row_matrix
+    offs = np.array(sorted([-o for o in offsets] + [0] + list(offsets)))
+    cols = np.arange(n)[:, None] + offs[None, :]
+    keep = (cols >= 0) & (cols < n)
+    vals = np.broadcast_to(np.where(offs == 0, 2.0 * len(offsets) + 0.5, -1.0), cols.shape)
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))])
+    return Compressed_row_matrix((n, n), rp, cols[keep].astype(np.int64), vals[keep])
+
+
+@pytest.mark.parametrize("left", [None, "jacobi"])
+@pytest.mark.parametrize("case", ["1", "33", "57", "ragged", "fits", "too wide"])
+def test_one_launch_cg_on_chip_and_not(gpu_lib, oracle, case, left):
+    """One-launch CG at the edges of its two forms.  With S CTAs a CTA of `per`
+    rows holds them on chip when per * (12 * width + 24) bytes fit 224 KB: 9
+    entries a row up to 1728 rows a CTA ("fits"); one row more gives CTAs of
+    1760 and the form that reads L2.  "ragged": CTAs of two slices, the last
+    ones without rows.  33 rows pad their slices too much for either form."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n, offs = {"1": (1, [1]), "33": (33, [1, 5]), "57": (57, [1, 5]), "ragged": (sms * 32 + 1, [1, 70]),
+               "fits": (sms * 1728, [1, 505, 506, 507]), "too wide": (sms * 1728 + 1, [1, 505, 506, 507])}[case]
+    A = _banded(n, offs)
+    b = oracle.spmv(A, matgen.uniform_vector(n, seed=3))
+    Ad = gpu.Device_matrix(A)
+    M = gpu.jacobi(Ad) if left else None
+    x = np.zeros(n)
+    before = _lib.launch_count()
+    s = gpu.conjugate_gradient(b, x, gpu.CGConfig(1e-10, 1000, 1000, True), gpu.spmv(Ad), M)
+    assert (_lib.launch_count() - before < 20) == (n != 33)
+    xr, sr = oracle.cg(A, b, np.zeros(n), 1e-10, 1000, 1000, left=left, collect=True)
+    assert s.converged and abs(s.computed_iterations - sr["computed_iterations"]) <= max(
+        1, sr["computed_iterations"] // 50)
+    k = min(s.computed_iterations, sr["computed_iterations"], 5)  # later ones differ by the sums' order
+    assert np.allclose(s.iteration_residuals[:k], sr["iteration_residuals"][:k], rtol=1e-10, atol=1e-14)
+    # true residuals of twice the tolerance at most, each; no eigenvalue below 0.5
+    assert np.linalg.norm(b - oracle.spmv(A, x)) <= 2e-10 * np.linalg.norm(b)
+    assert np.linalg.norm(x - xr) <= 8e-10 * np.linalg.norm(b)

@@ -96,3 +96,29 @@ def test_diagonal_copy_beside_it(gpu_lib, oracle, symmetric):
     y32 = torch.empty(n, dtype=torch.float32, device="cuda")
     Ad.spmv_f32(xd.float(), y32)
     assert np.array_equal(y32.cpu().numpy(), oracle.spmv(A.astype(np.float32), x.astype(np.float32)))
+
+
+def test_no_room_for_the_copy(gpu_lib, oracle):
+    """A device with room for the handle and half of its stencil copy: the handle
+    is made without it, holds nothing of it, and multiplies as before."""
+    import gc
+
+    import torch
+    A = matgen.laplacian_3d_dirichlet(128)
+    n = A.shape()[0]
+    full = gpu.Device_matrix(A)
+    assert full.layout() == "stencil"
+    size, copy = full.info()["device_bytes"], n * (4 * 8 + 2) + 64 + 128
+    full.close()
+    gc.collect()
+    torch.cuda.empty_cache()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - size + copy // 2, dtype=torch.uint8, device="cuda")
+    Ad = gpu.Device_matrix(A)
+    del held
+    torch.cuda.empty_cache()
+    assert Ad.layout() == "sell" and Ad.info()["device_bytes"] == size - copy
+    x = matgen.uniform_vector(n, seed=2)
+    xd = torch.from_numpy(x).cuda()
+    yd = torch.empty_like(xd)
+    Ad.spmv(xd, yd)
+    assert np.array_equal(yd.cpu().numpy(), oracle.spmv(A, x))
