@@ -851,7 +851,7 @@ def learned_runs(train_grid=128, instances=200, cycles=100, eval_grids=(128, 512
 def batched_runs(count=4096, loop_sample=64):
     """c5: `count` SPD systems (2-D 5-point / 3-D 7-point Laplacians plus a
     U[0, 0.5] shift, n log-uniform in [1k, 64k], FP32 CSR) solved to a 1e-10
-    FP64 residual in one persistent graph-captured launch with the
+    FP64 residual in one graph-captured call with the
     autotuned variant, against a loop of the plain FP64 Jacobi-CG solver
     over a seeded random sample of `loop_sample` systems (scaled to all)."""
     import torch

@@ -27,9 +27,9 @@ constexpr int kMaxRed = 4;       // fused reductions carried per kernel
 constexpr i64 kStencilMinEntries = 1 << 19;  // below, the products are bound by launch latency
 constexpr i64 kTileSmem = 192 * 1024;    // bytes of x in a CTA's shared memory
 // Fewest entries of the long rows.  Split against tiles, Zipf(1.5) rows of
-// random columns: FP64 34 against 45 us at 5.4M entries, 71 against 60 at 10.9M,
-// 144 against 94 at 22M, 437 against 228 at 69M; FP32 (whose x is half as far
-// beyond L1) 41 against 54 at 10.9M, 92 against 79 at 22M, 301 against 182 at 69M.
+// random columns: FP64 34 against 45 us at 5.4M entries, 72 against 56 at 10.9M,
+// 143 against 90 at 22M, 437 against 228 at 69M; FP32 (whose x is half as far
+// beyond L1) 41 against 54 at 10.9M, 93 against 80 at 22M, 301 against 183 at 69M.
 constexpr i64 kTileMinEntries64 = i64(8) << 20, kTileMinEntries32 = i64(16) << 20;
 constexpr i64 kTileSegment = 96;          // entries a long row should have in a panel
 constexpr int kSellMaxRow = 64;  // CSR rows up to this length use SELL-32
